@@ -564,7 +564,13 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
         for (uint32_t i = group; i < nit; i += ngroups) {
           uint32_t v, b0, b1;
           item_buckets(rg, __ldcg(items + i), v, b0, b1);
-          if (__ldcg(a.tpar + v) != kEmptyKey) continue;  // another chunk found one
+          // another chunk found one: other groups change the word, so it is
+          // read on one lane and broadcast -- read per lane, lanes of a group
+          // that drifted apart could disagree and wait for each other in the
+          // group-wide shuffles below for ever
+          uint32_t have = kEmptyKey;
+          if (L.gl == 0) have = __ldcg(a.tpar + v);
+          if (__shfl_sync(L.gmask, have, L.gbase) != kEmptyKey) continue;
           uint32_t found = kEmptyKey;
           for (uint32_t b = b0; b < b1 && found == kEmptyKey; ++b) {
             uint32_t sl = b;

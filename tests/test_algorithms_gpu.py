@@ -692,3 +692,28 @@ def test_bfs_repair_invalidates_only_vertices_whose_level_rises():
         assert inv_rep <= inv_plain
     for o in (plain, rep, G, Gr):
         o.close()
+
+
+def test_bfs_repair_with_hub_in_edges_in_many_work_items():
+    """Decremental BFS with a reverse graph whose hubs hold their in-edges in
+    many more buckets than one support-search item covers: several groups
+    look for the same candidate's new parent at once, and every group has to
+    act as one on what the others found.  Levels equal the oracle's."""
+    V = 1 << 12
+    s, d, _ = mk.gen_rmat(12, 120000, seed=211)
+    G, O = make_pair(V, s, d)
+    Gr = mk.DynamicGraph(V, degree_hints=degree_hints(d, V) * 64, reverse=True)
+    Gr.InsertEdges(to_dev(s), to_dev(d))
+    src = int(s[0])
+    bfs = mk.BFS(G, src, V)
+    bfs.set_reverse(Gr)
+    bfs.Static()
+    es = mk.EdgeSet(V, s, d)
+    for r in range(4):
+        ds, dd = es.sample_present(8000, seed=400 + r)
+        tds, tdd = to_dev(ds), to_dev(dd)
+        G.DeleteEdges(tds, tdd)
+        Gr.DeleteEdges(tds, tdd)
+        O.delete(ds, dd)
+        bfs.Decremental(tds, tdd)
+        np.testing.assert_array_equal(bfs.Distances(), O.bfs(src))
