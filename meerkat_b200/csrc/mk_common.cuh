@@ -115,29 +115,34 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p) {
 }
 
 // Grid-wide barrier for persistent kernels launched cooperatively (all
-// blocks co-resident).  bar[0] = arrival count, bar[1] = generation.  The
-// wait is bounded by `limit_ns`; on expiry the kernel's error word gets
-// kErrTimeout and the barrier returns false so every block can leave.
-__device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t *err,
-                                             unsigned long long limit_ns) {
-  __shared__ uint32_t ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t ok = 1;
-    uint32_t gen = ld_acquire_u32(bar + 1);
-    __threadfence();
-    uint32_t nblocks = gridDim.x * gridDim.y * gridDim.z;
-    uint32_t arrived = atomicAdd(bar, 1u);
-    if (arrived == nblocks - 1) {
-      atomicExch(bar, 0u);
+// blocks co-resident).  bar[0] counts arrivals and is zero at the launch; a
+// barrier is over once every block has arrived as often as this one, so an
+// arrival is one fire-and-forget add and nothing is reset between barriers
+// (the count wraps: compared as a signed difference).  One arrival and one
+// poller per block: launch few large blocks.  The wait is bounded by
+// `limit_ns`; on expiry the kernel's error word gets kErrTimeout and sync
+// returns false so every block can leave.
+struct GridBarrier {
+  uint32_t *bar, *err;
+  unsigned long long limit_ns;
+  uint32_t target = 0;  // arrivals that end the current barrier (thread 0)
+
+  __device__ __forceinline__ GridBarrier(uint32_t *b, uint32_t *e, unsigned long long limit)
+      : bar(b), err(e), limit_ns(limit) {}
+
+  __device__ __forceinline__ bool sync() {
+    __shared__ uint32_t ok_s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t ok = 1;
+      target += gridDim.x * gridDim.y * gridDim.z;
       __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
+      asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
       // the clock is read on every spin, so even a limit of a microsecond
       // is honoured; another block's timeout is noticed within 16 spins
       const unsigned long long t0 = global_ns();
       uint32_t spins = 0;
-      while (ld_acquire_u32(bar + 1) == gen) {
+      while ((int32_t)(ld_acquire_u32(bar) - target) < 0) {
         if (global_ns() - t0 > limit_ns) {
           atomicOr(err, kErrTimeout);
           ok = 0;
@@ -147,15 +152,14 @@ __device__ __forceinline__ bool grid_barrier(uint32_t *bar, uint32_t *err,
           ok = 0;
           break;
         }
-        __nanosleep(32);
       }
+      __threadfence();
+      ok_s = ok;
     }
-    __threadfence();
-    ok_s = ok;
+    __syncthreads();
+    return ok_s != 0;
   }
-  __syncthreads();
-  return ok_s != 0;
-}
+};
 
 // ---- TMA bulk copies and mbarriers (sm_90+ PTX, used on sm_100a) ----------
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {

@@ -70,7 +70,7 @@ __device__ __forceinline__ Kahan shfl_xor_kahan(const Kahan &k, uint32_t mask, i
   return r;
 }
 
-enum PrCtl : int { kPBar0 = 0, kPBar1 = 1, kPErr = 2, kPIters = 3, kPCur = 4, kPCtlWords = 8 };
+enum PrCtl : int { kPBar0 = 0, kPErr = 2, kPIters = 3, kPCur = 4, kPCtlWords = 8 };
 
 struct PrArgs {
   uint32_t V;
@@ -96,7 +96,7 @@ struct PrArgs {
   unsigned long long limit_ns;
 };
 
-constexpr int kPrBlock = 256;
+constexpr int kPrBlock = 512;  // three blocks per SM
 
 // Block reduction of two Kahan accumulators into part[..][blockIdx].
 __device__ __forceinline__ void block_reduce2(Kahan a, Kahan b, float *pa, float *pb) {
@@ -208,6 +208,7 @@ __global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
   auto pr = [&](uint32_t k) { return k ? a.pr1 : a.pr0; };
   auto cb = [&](uint32_t k) { return k ? a.c1 : a.c0; };
   auto part = [&](uint32_t parity, uint32_t kind) { return a.part + ((parity * 2 + kind) * 2) * nb; };
+  GridBarrier gb(a.ctl + kPBar0, a.ctl + kPErr, a.limit_ns);
   uint32_t cur = a.cur;
   const unsigned long long nitems = a.ioff[V], nmulti = a.moff[V];
   // this warp's run of 32-vertex groups: [glo, ghi), an equal share of the
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
       if (!od) dang.add(p);
     }
     block_reduce2(dang, zero, part(0, 0), part(0, 1));
-    if (!grid_barrier(a.ctl + kPBar0, a.ctl + kPErr, a.limit_ns)) return;
+    if (!gb.sync()) return;
   }
   uint32_t it = 0;
   float delta = 0.f, dangling = 0.f, unused = 0.f;
@@ -347,7 +348,7 @@ __global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
       }
     }
     if (nmulti) {
-      if (!grid_barrier(a.ctl + kPBar0, a.ctl + kPErr, a.limit_ns)) return;
+      if (!gb.sync()) return;
       // pass B: every hub combines its item partials in order
       for (unsigned long long m = wid; m < nmulti; m += nwarps) {
         const uint32_t u = a.multi[m];
@@ -365,7 +366,7 @@ __global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
       }
     }
     block_reduce2(kdang, kd, part(wp, 0), part(wp, 1));
-    if (!grid_barrier(a.ctl + kPBar0, a.ctl + kPErr, a.limit_ns)) return;
+    if (!gb.sync()) return;
     // this iteration's |delta| and the next one's dangling mass in one pass
     grid_totals(part(wp, 1), part(wp, 0), delta, dangling);
     cur ^= 1u;

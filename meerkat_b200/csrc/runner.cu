@@ -46,8 +46,8 @@ namespace mk {
 namespace {
 
 constexpr uint32_t kStepNone = 0, kStepBfs = 1, kStepWcc = 2;
-// ctl words of the one-launch step: grid barrier (count, generation), the
-// member counter; zeroed before every launch (a barrier that timed out
+// ctl words of the one-launch step: grid barrier arrivals, the member
+// counter; zeroed before every launch (a barrier that timed out
 // leaves its count behind)
 enum : int { kSBar0 = 0, kSMember = 2, kSCtlWords = 4 };
 
@@ -107,11 +107,12 @@ template <bool kW>
 __global__ void __launch_bounds__(kMemThreads, 1) k_set_step(GraphView g, StepArgs a) {
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_member, s_nfound, s_nitems;
+  GridBarrier gb(a.ctl + kSBar0, g.err, a.limit_ns);
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.count = 0;
   step_updates<kW, false>(g, a.ds, a.dd, nullptr, a.nd, nullptr, nullptr);
-  if (!grid_barrier(a.ctl + kSBar0, g.err, a.limit_ns)) return;
+  if (!gb.sync()) return;
   step_updates<kW, true>(g, a.is, a.id, a.iw, a.ni, a.applied, a.count);
-  if (!grid_barrier(a.ctl + kSBar0, g.err, a.limit_ns)) return;
+  if (!gb.sync()) return;
   const Lanes L = lanes();
   for (;;) {
     if (threadIdx.x == 0) s_member = atomicAdd(a.ctl + kSMember, 1u);
