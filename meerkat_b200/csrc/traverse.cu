@@ -54,15 +54,12 @@ enum TravMode : uint32_t { kStatic = 0, kIncremental = 1, kDecremental = 2 };
 enum Ctl : int {
   kBar0 = 0,      // barrier arrivals
   kErr = 2,       // sticky error bits
-  kThr = 3,       // near-far SSSP: distance threshold of the near frontier
   kSz0 = 4,       // frontier sizes kSz0 + (level % 3): words 4, 5, 6
   kRestart = 7,   // decremental: 1 when the call recomputed from the sources
   kInvCount = 8,  // invalidated vertices so far (append cursor of inv_list)
   kLevels = 9,    // relaxation levels run by the last call
   kDSz0 = 10,     // invalidation frontier sizes kDSz0 + (level % 3)
-  kFarN0 = 13,    // near-far SSSP: far list sizes kFarN0 + (list 0 / 1): words 13, 14
   kRound = 15,    // stamp base, persists across calls
-  kFarMin0 = 16,  // near-far SSSP: smallest distance on far list 0 / 1 (set in-kernel)
   kBegin = 18,    // blocks of the set-up kernel that are done (zero between launches)
   kTrimN = 20,    // BFS repair: seeds (heads of deleted tree edges)
   kTrimLo = 21,   // BFS repair: lowest / highest seed level
@@ -72,7 +69,9 @@ enum Ctl : int {
   kTChild = 27,   // BFS repair: child-scan items of the level
   kTReseed = 28,  // decremental with a reverse graph: re-seed items
   kEarly = 29,    // decremental: deleted tree edges counted before an immediate recompute
-  kCtlWords = 32
+  kFarN0 = 32,    // SSSP: far list sizes kFarN0 + (drain % 3): words 32, 33, 34
+  kFarMin0 = 35,  // SSSP: smallest distance pushed to that list: words 35, 36, 37 (set up as kNoFar)
+  kCtlWords = 40
 };
 constexpr uint32_t kRepairChunk = 8;  // buckets per repair / re-seed work item
 constexpr uint32_t kTrimMaxRounds = 256;  // BFS repair levels before a recompute
@@ -94,7 +93,7 @@ struct TravArgs {
   uint32_t nsources;
   uint32_t chunk;           // buckets per frontier work item
   uint32_t mode;
-  uint32_t delta;           // near-far SSSP step (0: plain level-synchronous)
+  uint32_t delta;           // near-far SSSP step (0: the threshold doubles)
   uint32_t recompute_inv;   // decremental: invalidated vertices from which to recompute (0: never)
   GraphView rg;             // in-edges of the same graph (static BFS pull levels), rg.V == 0: none
   uint32_t pull_items;      // static BFS: frontier size from which a level is pulled (0: never)
@@ -114,8 +113,10 @@ struct TravArgs {
 
 constexpr int kTravBlock = 1024;       // one block per SM: a grid barrier takes one arrival per block
 constexpr int kTravWarps = kTravBlock / 32;
-constexpr uint32_t kWarpQueue = 256;   // vertices a warp's queue holds
-constexpr uint32_t kWarpFlush = 128;   // vertices from which it is emptied between two rounds
+constexpr uint32_t kWarpQueue = 192;   // vertices a warp's queue holds
+constexpr uint32_t kWarpFlush = 96;    // vertices from which it is emptied between two rounds
+constexpr uint32_t kFarQueue = 160;    // the same for the far list (SSSP)
+constexpr uint32_t kFarFlush = 80;
 constexpr uint32_t kDefaultChunk = 4;  // buckets per frontier work item
 
 __host__ __device__ __forceinline__ unsigned long long item(uint32_t v, uint32_t chunk) {
@@ -232,17 +233,76 @@ __device__ __forceinline__ unsigned long long ld_dist(const unsigned long long *
 // Near-far split of static SSSP: an improved vertex whose new distance is
 // below `thr` joins the next level; otherwise it goes (once) onto the far
 // list, which is drained when the near frontier runs dry.  thr = kNoFar
-// sends everything to the next level.
+// sends everything to the next level.  Far pushes gather in a queue per warp
+// as the near ones do, with the smallest distance pushed.
 constexpr uint32_t kNoFar = 0xFFFFFFFFu;
+constexpr uint32_t kFarShift = 0;
 struct NearFar {
   uint32_t thr;
   uint32_t *far;   // list being appended
   uint32_t *farn;  // its size
+  uint32_t *farmin;  // smallest distance pushed to it
+  uint32_t *q;       // the warp's queue: kFarQueue vertex ids
+  uint32_t *qn;      // pushes since its last flush
+  uint32_t *qmin;    // smallest distance among them
 };
 
-__device__ __forceinline__ void far_push(const TravArgs &a, const NearFar &nf, uint32_t v) {
+// Appends v, at distance d, to the far list (it is on none).
+__device__ __forceinline__ void far_append(const NearFar &nf, uint32_t v, uint32_t d) {
+  const uint32_t pos = atomicAdd(nf.qn, 1u);
+  if (pos < kFarQueue) {
+    nf.q[pos] = v;
+    atomicMin(nf.qmin, d);
+  } else {
+    nf.far[atomicAdd(nf.farn, 1u)] = v;
+    atomicMin(nf.farmin, d);
+  }
+}
+
+__device__ __forceinline__ void far_push(const TravArgs &a, const NearFar &nf, uint32_t v, uint32_t d) {
   const uint32_t m = 1u << (v & 31);
-  if ((atomicOr(a.fbits + (v >> 5), m) & m) == 0) nf.far[atomicAdd(nf.farn, 1u)] = v;
+  if ((atomicOr(a.fbits + (v >> 5), m) & m) == 0) far_append(nf, v, d);
+}
+
+// Empties the warp's far queue into the list.  All 32 lanes call it together.
+__device__ __forceinline__ void far_flush(const NearFar &nf) {
+  const uint32_t lane = threadIdx.x & 31u;
+  __syncwarp();
+  const uint32_t n = min(*nf.qn, kFarQueue);
+  if (n) {
+    uint32_t base = 0;
+    if (lane == 0) {
+      base = atomicAdd(nf.farn, n);
+      atomicMin(nf.farmin, *nf.qmin);
+    }
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (uint32_t i = lane; i < n; i += 32) nf.far[base + i] = nf.q[i];
+  }
+  __syncwarp();
+  if (lane == 0) {
+    *nf.qn = 0u;
+    *nf.qmin = kNoFar;
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ bool far_full(const NearFar &nf) {
+  __syncwarp();
+  uint32_t n = 0;
+  if ((threadIdx.x & 31u) == 0) n = *nf.qn;
+  return __shfl_sync(0xFFFFFFFFu, n, 0) >= kFarFlush;
+}
+
+// Threshold of the next near phase, when the nearest far vertex is at
+// distance lo: a fixed step beyond it, or without one (delta == 0) twice its
+// distance.  Doubling needs no knowledge of the weights: on an R-MAT graph
+// most edges leave hubs a few units from the source, and phases [x, 2x) let
+// each of them expand about once (1.3 relaxations per edge instead of 5 when
+// every improvement expands at once, weights U[1, 1000]) in about twice the
+// levels; the number of phases is at most 32.
+__device__ __forceinline__ uint32_t next_threshold(uint32_t lo, uint32_t delta) {
+  const uint32_t step = delta ? delta : max(lo >> kFarShift, 1u);
+  return lo > kNoFar - step ? kNoFar : lo + step;
 }
 
 // Pushes v, whose distance just improved to nd, to the next level or the far list.
@@ -253,7 +313,7 @@ __device__ __forceinline__ void push_improved(const TravArgs &a, const WarpQueue
   if (nd < nf.thr) {
     if (atomicExch(a.stamp + v, stamp_next) != stamp_next) push_vertex(a, Q, v, gfr, gsz);
   } else {
-    far_push(a, nf, v);
+    far_push(a, nf, v, (uint32_t)nd);
   }
 }
 
@@ -479,8 +539,14 @@ template <bool kW, bool kUseW>
 __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
   __shared__ uint32_t q_s[kTravWarps][kWarpQueue];
   __shared__ uint32_t qn_s[kTravWarps];
+  __shared__ uint32_t fq_s[kUseW ? kTravWarps : 1][kFarQueue];
+  __shared__ uint32_t fqn_s[kTravWarps], fqmin_s[kTravWarps];
   const WarpQueue Q{q_s[threadIdx.x >> 5], qn_s + (threadIdx.x >> 5)};
-  if ((threadIdx.x & 31u) == 0) *Q.n = 0u;
+  if ((threadIdx.x & 31u) == 0) {
+    *Q.n = 0u;
+    fqn_s[threadIdx.x >> 5] = 0u;
+    fqmin_s[threadIdx.x >> 5] = kNoFar;
+  }
   __syncwarp();
   uint32_t npushed = 0;  // this warp's pushes
   const Lanes L = lanes();
@@ -494,14 +560,11 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
   GridBarrier gb(ctl + kBar0, err, a.limit_ns);
   unsigned long long *fr[2] = {a.fr0, a.fr1};
   const uint32_t round = ld_acquire_u32(ctl + kRound);
-  bool nearfar = kUseW && a.mode == kStatic && a.delta != 0 && a.far0 != nullptr;
-  const NearFar all_near{kNoFar, nullptr, nullptr};
-  uint32_t fb = 0;  // far list being appended
-  if (nearfar && tid == 0) {
-    ctl[kThr] = a.delta;
-    ctl[kFarMin0] = kNoFar;
-    ctl[kFarMin0 + 1] = kNoFar;
-  }
+  bool nearfar = kUseW && a.mode == kStatic;
+  const NearFar all_near{kNoFar, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  uint32_t fb = 0;     // far list being appended
+  uint32_t drain = 0;  // far lists drained so far, mod 3
+  uint32_t thr = a.delta ? a.delta : 1u;  // threshold of the near phase, the same in every thread
 
   // ---- seeding (level -1 pushes into fr[0] / sz[0]) ----
   if (a.mode == kStatic) {
@@ -773,12 +836,7 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
       // than re-seeding and repairing this many vertices.  The invalidation
       // bits are cleared in the epilogue as usual.
       for (uint32_t v = tid; v < a.g.V; v += nthreads) a.dist[v] = kInfInf;
-      if (tid == 0) {
-        ctl[kRestart] = 1u;
-        ctl[kThr] = a.delta;
-        ctl[kFarMin0] = kNoFar;
-        ctl[kFarMin0 + 1] = kNoFar;
-      }
+      if (tid == 0) ctl[kRestart] = 1u;
       if (!gb.sync()) return;
       for (uint32_t i = tid; i < a.nsources; i += nthreads) {
         const uint32_t src = a.sources[i];
@@ -790,7 +848,7 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
         for (uint32_t j = 0; j < k; ++j) a.fr0[base + j] = item(src, j);
         atomicAdd(a.pushed, 1ull);
       }
-      nearfar = kUseW && a.delta != 0 && a.far0 != nullptr;
+      nearfar = kUseW;
     } else if (hi > 0 && a.rg.V && a.treseed) {
       // D3 with the reverse graph: pull from each invalidated vertex's in-edges
       const uint32_t nri = ld_acquire_u32(ctl + kTReseed);
@@ -847,9 +905,12 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
 
   // ---- relaxation levels ----
   // A level expands the frontier; with near-far SSSP, a level whose frontier
-  // is empty instead drains the far list: the threshold moves to the far
-  // list's smallest distance plus delta, vertices below it join the next
-  // level and the rest move to the other far list.
+  // is empty instead drains the far list: the threshold moves beyond the
+  // smallest distance pushed to it, vertices below it join the next level and
+  // the rest move to the other far list.  A vertex that fell below the old
+  // threshold while it waited has been expanded since and is dropped.  The
+  // counters rotate over three words as the frontier sizes do: one is read,
+  // one filled, and the one read by the drain before is cleared.
   // The level loop ends when the frontier (and the far lists) run dry; as a
   // guard against a logic error that would keep it going with every barrier
   // met, a launch that has run longer than 64 wait limits (at least 60 s)
@@ -865,7 +926,7 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
     uint32_t nfar = 0;
     if (n == 0) {
       if (!nearfar) break;
-      nfar = ld_acquire_u32(ctl + kFarN0 + fb);
+      nfar = ld_acquire_u32(ctl + kFarN0 + drain);
       if (nfar == 0) break;
     }
     if (tid == 0) ctl[kSz0 + ((lv + 2) % 3)] = 0;
@@ -873,7 +934,6 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
     unsigned long long *nxt = fr[(lv + 1) & 1];
     uint32_t *nsz = ctl + kSz0 + ((lv + 1) % 3);
     const uint32_t stamp_next = round + 2 + lv;
-    const uint32_t thr = nearfar ? ld_acquire_u32(ctl + kThr) : kNoFar;
     if (n && !kUseW && a.mode == kStatic && a.pull_items && n >= a.pull_items) {
       // large BFS frontier: pull this level from the unvisited side
       if (a.rg.weighted)
@@ -881,7 +941,10 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
       else
         pull_level<false>(a, L, Q, group, ngroups, lv, stamp_next, nxt, nsz);
     } else if (n) {
-      const NearFar nf = nearfar ? NearFar{thr, fb ? a.far1 : a.far0, ctl + kFarN0 + fb} : all_near;
+      const NearFar nf = nearfar ? NearFar{thr, fb ? a.far1 : a.far0, ctl + kFarN0 + drain,
+                                           ctl + kFarMin0 + drain, fq_s[kUseW ? threadIdx.x >> 5 : 0],
+                                           fqn_s + (threadIdx.x >> 5), fqmin_s + (threadIdx.x >> 5)}
+                                 : all_near;
       // a warp's four groups take four consecutive items per round; the next
       // round's items are loaded ahead
       const uint32_t step = ngroups;
@@ -908,31 +971,40 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
           }
         }
         if (queue_full(Q)) npushed += queue_flush(a, Q, nxt, nsz);
+        if (kUseW && nearfar && far_full(nf)) far_flush(nf);
       }
+      if (kUseW && nearfar) far_flush(nf);
     } else {
       const uint32_t *fc = fb ? a.far1 : a.far0;
-      uint32_t *fo = fb ? a.far0 : a.far1;
-      for (uint32_t i = tid; i < nfar; i += nthreads)
-        atomicMin(ctl + kFarMin0 + fb, pack_hi(ld_dist(a.dist + __ldcg(fc + i))));
-      if (!gb.sync()) return;
-      const uint32_t lo = max(thr, ld_acquire_u32(ctl + kFarMin0 + fb));
-      const uint32_t nthr = lo > kNoFar - a.delta ? kNoFar : lo + a.delta;
-      for (uint32_t i = tid; i < nfar; i += nthreads) {
-        const uint32_t v = __ldcg(fc + i);
-        const uint32_t d = pack_hi(ld_dist(a.dist + v));
-        if (d < nthr) {
-          atomicAnd(a.fbits + (v >> 5), ~(1u << (v & 31)));
-          if (atomicExch(a.stamp + v, stamp_next) != stamp_next) push_vertex(a, Q, v, nxt, nsz);
-        } else {
-          fo[atomicAdd(ctl + kFarN0 + (fb ^ 1u), 1u)] = v;
-        }
-      }
+      const uint32_t into = drain == 2 ? 0u : drain + 1u;
+      const NearFar nf{thr, fb ? a.far0 : a.far1, ctl + kFarN0 + into, ctl + kFarMin0 + into,
+                       fq_s[kUseW ? threadIdx.x >> 5 : 0], fqn_s + (threadIdx.x >> 5),
+                       fqmin_s + (threadIdx.x >> 5)};
+      const uint32_t nthr = next_threshold(max(thr, ld_acquire_u32(ctl + kFarMin0 + drain)), a.delta);
       if (tid == 0) {
-        ctl[kThr] = nthr;
-        ctl[kFarN0 + fb] = 0;
-        // the other list's minimum is read by the next drain, not this one
-        ctl[kFarMin0 + (fb ^ 1u)] = kNoFar;
+        const uint32_t before = drain == 0 ? 2u : drain - 1u;
+        ctl[kFarN0 + before] = 0u;
+        ctl[kFarMin0 + before] = kNoFar;
       }
+      for (uint64_t w0 = tid - L.lane; w0 < nfar; w0 += nthreads) {
+        const uint64_t i = w0 + L.lane;
+        if (i < nfar) {
+          const uint32_t v = __ldcg(fc + i);
+          const uint32_t d = pack_hi(ld_dist(a.dist + v));
+          if (d >= nthr) {
+            far_append(nf, v, d);
+          } else {
+            atomicAnd(a.fbits + (v >> 5), ~(1u << (v & 31)));
+            if (d >= thr && atomicExch(a.stamp + v, stamp_next) != stamp_next)
+              push_vertex(a, Q, v, nxt, nsz);
+          }
+        }
+        if (queue_full(Q)) npushed += queue_flush(a, Q, nxt, nsz);
+        if (far_full(nf)) far_flush(nf);
+      }
+      far_flush(nf);
+      thr = nthr;
+      drain = into;
       fb ^= 1u;
     }
     npushed += queue_flush(a, Q, nxt, nsz);
@@ -1055,7 +1127,7 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (!last) return;
   const uint32_t i = threadIdx.x;
-  if (i < kCtlWords && i != kRound) ctl[i] = i == kTrimLo ? 0xFFFFFFFFu : 0u;
+  if (i < kCtlWords && i != kRound) ctl[i] = i == kTrimLo || (i >= kFarMin0 && i < kFarMin0 + 3) ? 0xFFFFFFFFu : 0u;
   if (i == kRound && recover) ctl[i] = 1u;
   if (i == kCtlWords) *pushed = 0ull;
 }
@@ -1163,8 +1235,7 @@ static void trav_begin(mk_traversal *t, bool fill, bool vis, bool fbits, cudaStr
 static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, const uint32_t *bd,
                             uint32_t n, cudaStream_t s, const uint32_t *srcs, uint32_t nsrc) {
   mk_graph *g = t->g;
-  const uint32_t delta = (t->sssp && mode != kIncremental && t->far0) ? g->tuning.sssp_delta : 0u;
-  trav_begin(t, mode == kStatic, mode == kStatic && t->vis, delta != 0, s);
+  trav_begin(t, mode == kStatic, mode == kStatic && t->vis, t->sssp && mode != kIncremental, s);
   TravArgs a;
   a.g = g->view();
   a.dist = t->dist;
@@ -1181,7 +1252,7 @@ static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, 
   a.sources = srcs ? srcs : t->sources;
   a.nsources = srcs ? nsrc : t->nsources;
   a.chunk = g->tuning.frontier_chunk ? g->tuning.frontier_chunk : kDefaultChunk;
-  a.delta = delta;
+  a.delta = g->tuning.sssp_delta;
   a.rg = t->rev ? t->rev->view() : GraphView{};
   if (!t->rev) a.rg.V = 0;
   a.pull_items = (t->rev && g->tuning.pull_permille)
