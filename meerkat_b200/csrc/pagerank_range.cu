@@ -10,12 +10,26 @@
 // range must be closed under out-edges.  Out-degrees are the graph's live
 // degrees, so a graph updated between calls needs no recount.
 //
-// One iteration: a dangling-mass reduction, a base fill of PR', a push pass
-// (one 8-lane group per bucket of the range, each live edge u -> v adds
-// PR[u] / outdeg[u] to PR'[v] with an FP64 atomic), and an |delta|
-// reduction read back by the host.  FP64 accumulation keeps the result
-// within the same L1 tolerance as the pull solver although the atomic order
-// varies from run to run.
+// A run first turns the range's live edges around: a counting sort by target
+// (count, scan, fill over the slabs) leaves the (source, target) pairs grouped
+// by target.  An iteration is then two launches:
+//   gather  a warp takes kPrrChunk consecutive pairs and sums d PR[u] / outdeg[u]
+//           over each target's run with segmented warp scans, so a target gets
+//           one FP64 atomic per run piece instead of one per edge, and a hub's
+//           run spreads over many warps;
+//   step    PR' per vertex, its next contribution, |delta| and the dangling
+//           mass of the next iteration.
+// What bounds it: the pairs stream from L2 (8 bytes an edge) and the gathers
+// of the contributions (8 bytes each, mostly L2).  Pushing straight from the
+// slabs (k_prr_push, kept for when the pairs do not fit in memory) walked
+// every 128-byte line and issued an atomic per edge in every iteration: 107 us
+// an iteration at 262,144 vertices and 4.1 M weighted edges, five launches and
+// a host round trip each.
+// The device decides when to stop: iterations are issued kPrrBatch at a time,
+// a launch behind the converged one returns at once, and the host reads the
+// deltas once per batch.  FP64 accumulation keeps the result within the same
+// L1 tolerance as the pull solver although the order of the sums varies from
+// run to run.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -89,6 +103,148 @@ __global__ void k_prr_push(GraphView g, uint32_t lo, uint32_t b0, uint32_t nb,
   }
 }
 
+constexpr uint32_t kPrrChunk = 512;  // pairs per warp of the gather
+constexpr uint32_t kPrrBatch = 12;   // iterations issued between two reads of the deltas
+constexpr uint32_t kPrrSteps = 4;    // 32-pair steps whose loads are in flight together
+
+// Live edges per target of the range (fill false), or the pairs written at
+// their targets' positions, the counts used up as cursors (fill true).  A key
+// outside the range (a range that is not closed under edges) is skipped and
+// reported as MK_DEVERR_INVALID_ID.
+template <bool kW, bool kFill>
+__global__ void k_prr_turn(GraphView g, uint32_t lo, uint32_t n, uint32_t b0, uint32_t nb,
+                           uint32_t *__restrict__ cnt, const unsigned long long *__restrict__ rp,
+                           uint2 *__restrict__ pairs) {
+  const Lanes L = lanes();
+  const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const uint32_t ngroups = (gridDim.x * blockDim.x) >> 3;
+  for (uint64_t i0 = (uint64_t)group * 4; i0 < nb; i0 += (uint64_t)ngroups * 4) {
+    const uint32_t b = b0 + (uint32_t)i0, m = nb - i0 < 4 ? (uint32_t)(nb - i0) : 4u;
+    const uint32_t own = kFill && L.gl < m ? __ldg(g.bowner + b + L.gl) - lo : 0u;
+    uint32_t src[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) src[j] = kFill ? __shfl_sync(L.gmask, own, L.gbase + j) : 0u;
+    walk4_levels(g, L, b, m, [&](uint32_t j, const uint4 q) {
+      const uint32_t u = j == 0 ? src[0] : j == 1 ? src[1] : j == 2 ? src[2] : src[3];
+      uint32_t k[4], w[4], at[4];
+      lane_keys<kW>(q, L.gl, k, w);
+#pragma unroll
+      for (int t = 0; t < keys_per_lane<kW>(); ++t) {
+        const uint32_t v = k[t] - lo;
+        if (k[t] >= kTombKey) {
+          k[t] = kEmptyKey;
+        } else if (k[t] < lo || v >= n) {
+          k[t] = kEmptyKey;
+          if (!kFill) atomicOr(g.err, kErrInvalidId);
+        } else if (!kFill) {
+          atomicAdd(cnt + v, 1u);
+        } else {
+          const uint32_t left = atomicSub(cnt + v, 1u);
+          at[t] = left - 1u;
+          if (left == 0) k[t] = kEmptyKey;  // not counted: the graph changed under the call
+        }
+      }
+      if (!kFill) return;
+#pragma unroll
+      for (int t = 0; t < keys_per_lane<kW>(); ++t)
+        if (k[t] != kEmptyKey) pairs[rp[k[t] - lo] + at[t]] = make_uint2(u, k[t] - lo);
+    });
+  }
+}
+
+// PR = x, the first contributions, empty sums, the first dangling mass.
+__global__ void k_prr_start(double *__restrict__ pr, double *__restrict__ c, double *__restrict__ sum,
+                            const uint32_t *__restrict__ deg, uint32_t n, double x, double d,
+                            double *dang) {
+  double lost = 0.0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t dg = deg[i];
+    pr[i] = x;
+    sum[i] = 0.0;
+    c[i] = dg ? d * x / (double)dg : 0.0;
+    if (!dg) lost += x;
+  }
+  block_add(lost, dang);
+}
+
+// Whether the iteration before this one (its |delta| in *before; null: none)
+// ended the solve.  An iteration that did not run leaves its delta at zero,
+// so every later one sees it as ended too.
+__device__ __forceinline__ bool prr_done(const double *before, double d, double stop) {
+  return before && *before * d / (1.0 - d) <= stop;
+}
+
+__global__ void __launch_bounds__(256)
+    k_prr_gather(const uint2 *__restrict__ pairs, unsigned long long E, const double *__restrict__ c,
+                 double *sum, const double *before, double d, double stop) {
+  if (prr_done(before, d, stop)) return;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+  for (uint64_t e0 = warp * kPrrChunk; e0 < E; e0 += nwarps * kPrrChunk) {
+    const uint64_t e1 = e0 + kPrrChunk < E ? e0 + kPrrChunk : E;
+    uint32_t ckey = kEmptyKey;  // target whose run is open, and its sum so far
+    double cval = 0.0;
+    for (uint64_t s0 = e0; s0 < e1; s0 += 32u * kPrrSteps) {
+      uint2 p[kPrrSteps];
+      double val[kPrrSteps];
+#pragma unroll
+      for (uint32_t r = 0; r < kPrrSteps; ++r) {
+        const uint64_t e = s0 + 32u * r + lane;
+        p[r] = e < e1 ? __ldg(pairs + e) : make_uint2(0u, kEmptyKey);
+      }
+#pragma unroll
+      for (uint32_t r = 0; r < kPrrSteps; ++r) val[r] = p[r].y != kEmptyKey ? __ldg(c + p[r].x) : 0.0;
+#pragma unroll
+      for (uint32_t r = 0; r < kPrrSteps; ++r) {
+        const uint32_t key = p[r].y;
+        double v = val[r];
+        const uint32_t first = __shfl_sync(0xFFFFFFFFu, key, 0);
+        if (first == kEmptyKey) break;  // past the end (uniform)
+        if (lane == 0) {
+          if (key == ckey)
+            v += cval;
+          else if (ckey != kEmptyKey)
+            atomicAdd(sum + ckey, cval);
+        }
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xFFFFFFFFu, v, o);
+          const uint32_t ky = __shfl_up_sync(0xFFFFFFFFu, key, o);
+          if (lane >= o && ky == key) v += y;
+        }
+        const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, key, 1);
+        if (lane < 31 && key != next && key != kEmptyKey) atomicAdd(sum + key, v);
+        ckey = __shfl_sync(0xFFFFFFFFu, key, 31);  // empty when the chunk ended in this step
+        cval = __shfl_sync(0xFFFFFFFFu, v, 31);
+      }
+    }
+    if (lane == 0 && ckey != kEmptyKey) atomicAdd(sum + ckey, cval);
+  }
+}
+
+// PR' from the gathered sums (emptied again), the next contributions;
+// *delta += |PR' - PR|, dang[1] += the dangling mass of PR'.
+__global__ void __launch_bounds__(256)
+    k_prr_step(double *__restrict__ pr, double *__restrict__ c, double *__restrict__ sum,
+               const uint32_t *__restrict__ deg, uint32_t n, double *dang, double *delta,
+               const double *before, double d, double stop) {
+  if (prr_done(before, d, stop)) return;
+  const double base = (1.0 - d) / n + d * dang[0] / n;
+  double moved = 0.0, lost = 0.0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double nv = base + sum[i];
+    const uint32_t dg = deg[i];
+    moved += fabs(nv - pr[i]);
+    pr[i] = nv;
+    sum[i] = 0.0;
+    c[i] = dg ? d * nv / (double)dg : 0.0;
+    if (!dg) lost += nv;
+  }
+  block_add(moved, delta);
+  block_add(lost, dang + 1);
+}
+
 // acc[1] += sum |nx - pr|
 __global__ void k_prr_delta(const double *__restrict__ pr, const double *__restrict__ nx,
                             uint32_t n, double *acc) {
@@ -116,7 +272,13 @@ struct mk_pagerank_range {
   mk_graph *g = nullptr;
   uint32_t cap = 0;  // vertices
   double *a = nullptr, *b = nullptr;
-  double *acc = nullptr;  // [0] dangling, [1] delta
+  // push form: [0] dangling, [1] delta; else the dangling mass before every
+  // iteration of a batch and after it, then the iterations' deltas
+  double *acc = nullptr;
+  DevBuf<uint2> pairs;  // (source, target) of every live edge, by target
+  DevBuf<double> c;     // contributions d PR / outdeg
+  DevBuf<uint32_t> cnt;
+  DevBuf<unsigned long long> rp, tmp;
   float *out = nullptr;
   uint32_t n = 0;  // vertices of the last run
   uint32_t iters = 0;
@@ -137,7 +299,7 @@ mk_status mk_pagerank_range_create(mk_graph *g, uint32_t max_vertices, mk_pagera
   p->cap = max_vertices;
   cudaError_t e = cudaMalloc(&p->a, (size_t)max_vertices * 8);
   if (e == cudaSuccess) e = cudaMalloc(&p->b, (size_t)max_vertices * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&p->acc, 16);
+  if (e == cudaSuccess) e = cudaMalloc(&p->acc, (2 * kPrrBatch + 1) * 8);
   if (e == cudaSuccess) e = cudaMalloc(&p->out, (size_t)max_vertices * 4);
   if (e != cudaSuccess) {
     mk_pagerank_range_destroy(p);
@@ -146,6 +308,80 @@ mk_status mk_pagerank_range_create(mk_graph *g, uint32_t max_vertices, mk_pagera
   *out = p;
   return MK_OK;
 }
+
+}  // extern "C"
+
+// Turns the range's edges around (p->pairs); *edges their number.  MK_ERR_OOM
+// when they do not fit.
+static mk_status prr_turn(mk_pagerank_range *p, uint32_t lo, uint32_t n, uint32_t b0, uint32_t nb,
+                          cudaStream_t s, unsigned long long *edges) {
+  mk_graph *g = p->g;
+  MK_CHECK(p->cnt.reserve(n));
+  MK_CHECK(p->rp.reserve((size_t)n + 1));
+  MK_CHECK(p->c.reserve(n));
+  const GraphView v = g->view();
+  const int gb = (int)std::min<uint64_t>((uint64_t)nb * 2 / 256 + 1, (uint64_t)device_sm_count(g->device) * 8);
+  MK_CUDA(cudaMemsetAsync(p->cnt.ptr, 0, (size_t)n * 4, s));
+  if (g->weighted)
+    k_prr_turn<true, false><<<gb, 256, 0, s>>>(v, lo, n, b0, nb, p->cnt.ptr, nullptr, nullptr);
+  else
+    k_prr_turn<false, false><<<gb, 256, 0, s>>>(v, lo, n, b0, nb, p->cnt.ptr, nullptr, nullptr);
+  MK_CHECK(scan_u32_to_u64(p->cnt.ptr, p->rp.ptr, n, p->tmp, s));
+  MK_CUDA(cudaMemcpyAsync(edges, p->rp.ptr + n, 8, cudaMemcpyDeviceToHost, s));
+  MK_CUDA(cudaStreamSynchronize(s));
+  MK_CHECK(p->pairs.reserve(std::max<unsigned long long>(*edges, 1)));
+  if (g->weighted)
+    k_prr_turn<true, true><<<gb, 256, 0, s>>>(v, lo, n, b0, nb, p->cnt.ptr, p->rp.ptr, p->pairs.ptr);
+  else
+    k_prr_turn<false, true><<<gb, 256, 0, s>>>(v, lo, n, b0, nb, p->cnt.ptr, p->rp.ptr, p->pairs.ptr);
+  MK_CUDA(cudaGetLastError());
+  return MK_OK;
+}
+
+// The iterations over the turned edges; the ranks end in p->a.
+static mk_status prr_gather_solve(mk_pagerank_range *p, uint32_t lo, uint32_t n, unsigned long long E,
+                                  double d, double stop, uint32_t max_iter, cudaStream_t s,
+                                  uint32_t *iters, double *last) {
+  mk_graph *g = p->g;
+  const uint32_t *deg = g->deg + lo;
+  const int fb = flat_blocks(n, g->device);
+  const uint64_t chunks = (E + kPrrChunk - 1) / kPrrChunk;
+  const int eb = (int)std::max<uint64_t>(
+      1, std::min<uint64_t>((chunks + 7) / 8, (uint64_t)device_sm_count(g->device) * 8));
+  double *dang = p->acc, *delta = p->acc + kPrrBatch + 1;
+  MK_CUDA(cudaMemsetAsync(p->acc, 0, (2 * kPrrBatch + 1) * 8, s));
+  k_prr_start<<<fb, 256, 0, s>>>(p->a, p->c.ptr, p->b, deg, n, 1.0 / n, d, dang);
+  MK_CUDA(cudaGetLastError());
+  uint32_t it = 0;
+  double h[kPrrBatch];
+  while (it < max_iter) {
+    const uint32_t k = std::min(kPrrBatch, max_iter - it);
+    for (uint32_t i = 0; i < k; ++i) {
+      const double *before = i ? delta + i - 1 : nullptr;
+      k_prr_gather<<<eb, 256, 0, s>>>(p->pairs.ptr, E, p->c.ptr, p->b, before, d, stop);
+      k_prr_step<<<fb, 256, 0, s>>>(p->a, p->c.ptr, p->b, deg, n, dang + i, delta + i, before, d, stop);
+    }
+    MK_CUDA(cudaGetLastError());
+    MK_CUDA(cudaMemcpyAsync(h, delta, sizeof(double) * k, cudaMemcpyDeviceToHost, s));
+    MK_CUDA(cudaStreamSynchronize(s));
+    for (uint32_t i = 0; i < k; ++i) {
+      ++it;
+      *last = h[i];
+      if (h[i] * d / (1.0 - d) <= stop) {
+        *iters = it;
+        return MK_OK;
+      }
+    }
+    if (it < max_iter) {  // the next batch starts from the dangling mass this one left
+      MK_CUDA(cudaMemcpyAsync(dang, dang + kPrrBatch, 8, cudaMemcpyDeviceToDevice, s));
+      MK_CUDA(cudaMemsetAsync(dang + 1, 0, 2 * kPrrBatch * 8, s));
+    }
+  }
+  *iters = it;
+  return MK_OK;
+}
+
+extern "C" {
 
 mk_status mk_pagerank_range_run(mk_pagerank_range *p, uint32_t v_begin, uint32_t v_end,
                                 float damping, float tol, uint32_t max_iter, void *stream,
@@ -168,24 +404,34 @@ mk_status mk_pagerank_range_run(mk_pagerank_range *p, uint32_t v_begin, uint32_t
   const int gb = (int)std::min<uint64_t>((uint64_t)nb * 8 / 256 + 1, (uint64_t)device_sm_count(g->device) * 8);
   const GraphView v = g->view();
   double *pr = p->a, *nx = p->b;
-  k_prr_fill<<<fb, 256, 0, s>>>(pr, n, 1.0 / n);
   uint32_t it = 0;
   double delta = 0.0;
-  while (it < max_iter) {
-    MK_CUDA(cudaMemsetAsync(p->acc, 0, 16, s));
-    k_prr_dangling<<<fb, 256, 0, s>>>(pr, g->deg + v_begin, n, p->acc);
-    k_prr_base<<<fb, 256, 0, s>>>(nx, n, p->acc, d);
-    if (g->weighted)
-      k_prr_push<true><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
-    else
-      k_prr_push<false><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
-    k_prr_delta<<<fb, 256, 0, s>>>(pr, nx, n, p->acc);
-    MK_CUDA(cudaGetLastError());
-    MK_CUDA(cudaMemcpyAsync(&delta, p->acc + 1, 8, cudaMemcpyDeviceToHost, s));
-    MK_CUDA(cudaStreamSynchronize(s));
-    std::swap(pr, nx);
-    ++it;
-    if (delta * d / (1.0 - d) <= 0.5 * tol) break;
+  unsigned long long E = 0;
+  const mk_status turned = prr_turn(p, v_begin, n, b0, nb, s, &E);
+  if (turned == MK_OK) {
+    MK_CHECK(prr_gather_solve(p, v_begin, n, E, d, 0.5 * tol, max_iter, s, &it, &delta));
+  } else if (turned != MK_ERR_OOM) {
+    return turned;
+  } else {
+    // the pairs do not fit beside what the process holds: push from the slabs
+    (void)cudaGetLastError();
+    k_prr_fill<<<fb, 256, 0, s>>>(pr, n, 1.0 / n);
+    while (it < max_iter) {
+      MK_CUDA(cudaMemsetAsync(p->acc, 0, 16, s));
+      k_prr_dangling<<<fb, 256, 0, s>>>(pr, g->deg + v_begin, n, p->acc);
+      k_prr_base<<<fb, 256, 0, s>>>(nx, n, p->acc, d);
+      if (g->weighted)
+        k_prr_push<true><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
+      else
+        k_prr_push<false><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
+      k_prr_delta<<<fb, 256, 0, s>>>(pr, nx, n, p->acc);
+      MK_CUDA(cudaGetLastError());
+      MK_CUDA(cudaMemcpyAsync(&delta, p->acc + 1, 8, cudaMemcpyDeviceToHost, s));
+      MK_CUDA(cudaStreamSynchronize(s));
+      std::swap(pr, nx);
+      ++it;
+      if (delta * d / (1.0 - d) <= 0.5 * tol) break;
+    }
   }
   k_prr_out<<<fb, 256, 0, s>>>(pr, n, p->out);
   MK_CUDA(cudaGetLastError());
@@ -217,6 +463,11 @@ mk_status mk_pagerank_range_destroy(mk_pagerank_range *p) {
   cudaFree(p->b);
   cudaFree(p->acc);
   cudaFree(p->out);
+  p->pairs.release();
+  p->c.release();
+  p->cnt.release();
+  p->rp.release();
+  p->tmp.release();
   delete p;
   return MK_OK;
 }
