@@ -189,15 +189,11 @@ __device__ __forceinline__ void ls_union(uint16_t *p, uint32_t a, uint32_t b, ui
   atomicOr(err, kErrTimeout);
 }
 
-// R = (first vertex, end vertex, first bucket, end bucket), at most
-// kUfLocalMax vertices; labels[R.x .. R.y) get the minimum vertex id of each
-// component.  A key outside the range (a range that is not closed under
-// edges) is skipped and reported as MK_DEVERR_INVALID_ID.  sp holds
-// uf_member_smem(n) bytes.  Ends with the CTA synchronised.
+// The unions of buckets [R.z, R.w), which are the range's or a part of them,
+// over the range's own sets.  Ends with the CTA synchronised.
 template <bool kW, bool kFused>
-__device__ __forceinline__ void uf_member(const GraphView &g, const Lanes &L, const uint4 R,
-                                          uint32_t *__restrict__ labels, uint32_t *err,
-                                          uint16_t *sp) {
+__device__ __forceinline__ void uf_member_link(const GraphView &g, const Lanes &L, const uint4 R,
+                                               uint32_t *err, uint16_t *sp) {
   const uint32_t group = threadIdx.x >> 3, ngroups = blockDim.x >> 3;
   const uint32_t lo = R.x, n = R.y - R.x;
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) sp[i] = (uint16_t)i;
@@ -224,8 +220,64 @@ __device__ __forceinline__ void uf_member(const GraphView &g, const Lanes &L, co
     });
   }
   __syncthreads();
+}
+
+// Every vertex's root as its label.  Ends with the CTA synchronised.
+__device__ __forceinline__ void uf_member_labels(const uint4 R, uint32_t *__restrict__ labels,
+                                                 const uint16_t *sp) {
+  const uint32_t lo = R.x, n = R.y - R.x;
   for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) labels[lo + i] = lo + ls_root(sp, i);
   __syncthreads();
+}
+
+// A range's parts, solved by P CTAs (a power of two) that never wait for one
+// another: the sets of the parts are joined in a tournament.  A CTA that
+// finishes a subtree writes its sets (a root per vertex) to the subtree's
+// slot and counts itself at the parent node; the first of the two to arrive
+// leaves, the second joins the other's sets into its own and goes on.  True
+// in the one CTA that ends with the sets of the whole range.  slots: P arrays
+// of `stride` words, flags: P counters, zero before the launch.
+__device__ __forceinline__ bool uf_member_join(uint32_t n, uint32_t part, uint32_t P, uint32_t stride,
+                                               uint16_t *slots, uint32_t *flags, uint16_t *sp,
+                                               uint32_t *err) {
+  __shared__ uint32_t s_second;
+  for (uint32_t l = 1; l < P; l <<= 1) {
+    const uint32_t base = part & ~(2 * l - 1);           // first part below the parent node
+    const uint32_t mine = base + ((part & l) ? l : 0u);  // slot of this CTA's subtree
+    uint16_t *out = slots + (size_t)mine * stride;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) out[i] = (uint16_t)ls_root(sp, i);
+    __threadfence();
+    __syncthreads();
+    // node (l, base): base + l is a different index for every node of a range
+    if (threadIdx.x == 0) {
+      s_second = atomicAdd(flags + base + l, 1u);
+      __threadfence();
+    }
+    __syncthreads();
+    const bool second = s_second != 0;
+    __syncthreads();
+    if (!second) return false;
+    const uint16_t *other = slots + (size_t)(mine == base ? base + l : base) * stride;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+      const uint32_t r = __ldcg(reinterpret_cast<const unsigned short *>(other + i));
+      if (r != i) ls_union(sp, i, r, err);
+    }
+    __syncthreads();
+  }
+  return true;
+}
+
+// R = (first vertex, end vertex, first bucket, end bucket), at most
+// kUfLocalMax vertices; labels[R.x .. R.y) get the minimum vertex id of each
+// component.  A key outside the range (a range that is not closed under
+// edges) is skipped and reported as MK_DEVERR_INVALID_ID.  sp holds
+// uf_member_smem(n) bytes.  Ends with the CTA synchronised.
+template <bool kW, bool kFused>
+__device__ __forceinline__ void uf_member(const GraphView &g, const Lanes &L, const uint4 R,
+                                          uint32_t *__restrict__ labels, uint32_t *err,
+                                          uint16_t *sp) {
+  uf_member_link<kW, kFused>(g, L, R, err, sp);
+  uf_member_labels(R, labels, sp);
 }
 
 }  // namespace mk

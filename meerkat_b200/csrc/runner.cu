@@ -148,6 +148,10 @@ struct mk_set_runner {
   uint32_t *sctl = nullptr;
   size_t ssmem = 0;
   int sgrid = 0;
+  // the sequence's components run beside its BFS: a stream of the runner's
+  // own, forked from the caller's after the updates and joined to it again
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
 };
 
 namespace {
@@ -251,6 +255,15 @@ mk_status mk_set_runner_create(mk_graphset *s, const uint8_t *h_query,
     st = mk_wcc_create(g, &r->wcc);
     if (st == MK_OK) st = mk_wcc_prepare_ranges(r->wcc, wcc_ranges.data(), r->n_wcc);
   }
+  if (st == MK_OK && r->bfs && r->wcc && max_member <= kMemLocalMax) {
+    // (larger members go through device-wide kernels, one of them a
+    // cooperative launch that needs every SM: no room beside it)
+    DeviceGuard dg(g->device);
+    cudaError_t e = cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->join, cudaEventDisableTiming);
+    if (e != cudaSuccess) st = cuda_fail(e, "mk_set_runner_create: side stream");
+  }
   if (st == MK_OK && max_member <= kMemLocalMax && !g->reverse) {
     DeviceGuard dg(g->device);
     st = build_single(r, off, h_query, h_bfs_source_local);
@@ -331,6 +344,21 @@ mk_status mk_set_runner_step(mk_set_runner *r, const uint32_t *d_del_src,
   }
   MK_CHECK(mk_graph_delete_edges(r->g, d_del_src, d_del_dst, n_del, stream));
   MK_CHECK(mk_graph_insert_edges(r->g, d_ins_src, d_ins_dst, d_ins_w, n_ins, stream));
+  if (r->side) {
+    // Both query kernels end in a tail of few busy SMs (a member per CTA, an
+    // eightfold spread of sizes); side by side each fills the other's.  They
+    // share only the graph, which neither writes.
+    DeviceGuard dg(r->g->device);
+    cudaStream_t s = as_stream(stream);
+    MK_CUDA(cudaEventRecord(r->fork, s));
+    MK_CUDA(cudaStreamWaitEvent(r->side, r->fork, 0));
+    const mk_status bs = mk_bfs_static_members(r->bfs, stream, nullptr);
+    const mk_status ws = mk_wcc_static_prepared(r->wcc, r->side, nullptr);
+    // joined whatever happened: the caller's stream stays ordered behind both
+    MK_CUDA(cudaEventRecord(r->join, r->side));
+    MK_CUDA(cudaStreamWaitEvent(s, r->join, 0));
+    return bs != MK_OK ? bs : ws;
+  }
   if (r->bfs) MK_CHECK(mk_bfs_static_members(r->bfs, stream, nullptr));
   if (r->wcc) MK_CHECK(mk_wcc_static_prepared(r->wcc, stream, nullptr));
   return MK_OK;
@@ -356,6 +384,9 @@ mk_status mk_set_runner_destroy(mk_set_runner *r) {
   if (r->wcc) mk_wcc_destroy(r->wcc);
   r->stab.release();
   if (r->sctl) cudaFree(r->sctl);
+  if (r->join) cudaEventDestroy(r->join);
+  if (r->fork) cudaEventDestroy(r->fork);
+  if (r->side) cudaStreamDestroy(r->side);
   delete r;
   return MK_OK;
 }

@@ -1078,7 +1078,7 @@ struct mk_traversal {
   size_t rcap = 0;  // re-seed / support item capacity
   std::vector<uint32_t> h_sources;
   // prepared member table (BFS): counter word, uint4 (lo, hi, b0, b1) per
-  // small range (largest first), their sources, then the sources whose
+  // small range (most buckets first), their sources, then the sources whose
   // range is too large for shared memory
   DevBuf<uint32_t> members;
   uint32_t n_small = 0, n_large = 0, small_max = 0;
@@ -1455,8 +1455,13 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
     if (spans[i].first < spans[i - 1].second)
       return fail(MK_ERR_INVALID, std::string(what) + ": overlapping ranges");
   auto len = [&](uint32_t r) { return h_vertex_ranges[2 * r + 1] - h_vertex_ranges[2 * r]; };
+  auto buckets = [&](uint32_t r) {
+    return g->h_boff[h_vertex_ranges[2 * r + 1]] - g->h_boff[h_vertex_ranges[2 * r]];
+  };
+  // the largest first by what a CTA walks, not by vertices: average degrees
+  // differ eightfold between members
   std::stable_sort(small_ids.begin(), small_ids.end(),
-                   [&](uint32_t a, uint32_t b) { return len(a) > len(b); });
+                   [&](uint32_t a, uint32_t b) { return buckets(a) > buckets(b); });
   const size_t ns = small_ids.size(), nl = large_src.size();
   std::vector<uint32_t> host(4 + 5 * ns + nl, 0u);
   uint32_t *tab = host.data() + 4, *ssrc = tab + 4 * ns, *lsrc = ssrc + ns;
@@ -1477,7 +1482,8 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   MK_CUDA(cudaMemcpy(t->members.ptr, host.data(), host.size() * 4, cudaMemcpyHostToDevice));
   t->n_small = (uint32_t)ns;
   t->n_large = (uint32_t)nl;
-  t->small_max = ns ? len(small_ids[0]) : 0;
+  t->small_max = 0;
+  for (uint32_t r : small_ids) t->small_max = std::max(t->small_max, len(r));
   t->small_grid = 0;
   if (ns) {
     const size_t smem = bfs_member_smem(t->small_max);

@@ -103,7 +103,7 @@ __device__ __forceinline__ void uf_union(uint32_t *p, uint32_t a, uint32_t b, ui
 // the call (kEmptyKey when the retry limit ran out).  An edge pass keeps it
 // as the owner's parent for the owner's next keys: a key whose parent equals
 // it is in the same set, so the hook just made is not tried again key by key.
-__device__ __forceinline__ uint32_t uf_union_root(uint32_t *p, uint32_t a, uint32_t b,
+__device__ __noinline__ uint32_t uf_union_root(uint32_t *p, uint32_t a, uint32_t b,
                                                   uint32_t *err, unsigned long long *fe) {
   for (uint32_t it = 0; it < kUfLimit; ++it) {
     const uint32_t ra = uf_find(p, a), rb = uf_find(p, b);
@@ -256,19 +256,26 @@ __device__ __forceinline__ void link_bucket_skip(const GraphView &g, const Lanes
 // loaded together, chains are followed level by level, and a lane loads the
 // parents of all its keys before comparing, so one group keeps several
 // reads in flight instead of one dependent read per key.
+// With `big` (k_uf_big_bits, which stand during the pass) an edge with both
+// ends in the big set is skipped on its key's bit alone: a bit is 32 times
+// denser than a parent word, so most tests hit L1, and on a graph with a
+// giant component 99 % of the edges end there (48 M edges: 805 us reading
+// every key's parent through L2, see the static passes for the rest).
 template <bool kW>
 __global__ void k_uf_edges_skip(GraphView g, uint32_t *p, const uint32_t *sel_bits, uint32_t *err,
-                                unsigned long long *fe, const unsigned long long *skip_if = nullptr) {
+                                unsigned long long *fe, const unsigned long long *skip_if = nullptr,
+                                const uint32_t *__restrict__ big = nullptr) {
   if (skip_if && *skip_if) return;
   const Lanes L = lanes();
   const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
   const uint32_t ngroups = (gridDim.x * blockDim.x) >> 3;
   for (uint64_t b0 = (uint64_t)group * 4; b0 < g.nbuckets; b0 += (uint64_t)ngroups * 4) {
     const uint32_t b = (uint32_t)b0, m = min(4u, g.nbuckets - b);
-    uint32_t own[4], pu[4], live = 0;
+    uint32_t own[4], pu[4], live = 0, inbig = 0;
 #pragma unroll
     for (uint32_t j = 0; j < 4; ++j) {
       own[j] = j < m ? __ldg(g.bowner + b + j) : 0u;
+      if (big && j < m) inbig |= ((__ldg(big + (own[j] >> 5)) >> (own[j] & 31)) & 1u) << j;
       const bool ok = j < m && g.deg[own[j]] != 0 &&
                       (!sel_bits || ((sel_bits[own[j] >> 5] >> (own[j] & 31)) & 1u));
       live |= (ok ? 1u : 0u) << j;
@@ -287,6 +294,11 @@ __global__ void k_uf_edges_skip(GraphView g, uint32_t *p, const uint32_t *sel_bi
 #pragma unroll
       for (int t = 0; t < keys_per_lane<kW>(); ++t) {
         ok[t] = k[t] < kTombKey && k[t] != u;
+        pv[t] = ((inbig >> j) & 1u) && ok[t] ? __ldg(big + (k[t] >> 5)) : 0u;
+      }
+#pragma unroll
+      for (int t = 0; t < keys_per_lane<kW>(); ++t) {
+        ok[t] = ok[t] && !((pv[t] >> (k[t] & 31)) & 1u);
         pv[t] = ok[t] ? __ldcg(p + k[t]) : 0u;
       }
 #pragma unroll
@@ -312,7 +324,8 @@ enum : int {
   kFGiant = 7,      // static passes: the most sampled set's root + 1 (0: none)
   kFItemsOut = 8,   // scan items listed for the graph (out-edges)
   kFItemsIn = 9,    // scan items listed for the reverse graph (in-edges)
-  kFCtlWords = 10
+  kFBig = 10,       // static passes: the root of the most frequent sampled set + 1 (0: under 1/8 of the samples)
+  kFCtlWords = 11
 };
 
 // A scan item is the first of up to kItemBuckets consecutive buckets of one
@@ -671,6 +684,23 @@ __global__ void __launch_bounds__(kMainThreads)
   if (threadIdx.x == 0)
     ctl[kFGiant] = ((best >> 32) >= 32 && 4 * (best >> 32) >= 3ull * drawn)
                        ? (unsigned long long)(uint32_t)best + 1 : 0ull;
+  if (threadIdx.x == 0)
+    ctl[kFBig] = ((best >> 32) >= 32 && 8 * (best >> 32) >= (unsigned long long)drawn)
+                     ? (unsigned long long)(uint32_t)best + 1 : 0ull;
+}
+
+// Bit per vertex: its (compressed) parent is the big set's root.  All zero
+// without a big set.
+__global__ void k_uf_big_bits(const uint32_t *p, uint32_t V, const unsigned long long *ctl,
+                              uint32_t *__restrict__ bits) {
+  const unsigned long long big = ctl[kFBig];
+  const uint32_t words = (V + 31) / 32, lane = threadIdx.x & 31u;
+  const uint32_t stride = gridDim.x * blockDim.x;  // a multiple of 32
+  for (uint64_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < words * 32ull; base += stride) {
+    const uint64_t x = base + lane;
+    const uint32_t word = __ballot_sync(0xFFFFFFFFu, big && x < V && __ldcg(p + x) == (uint32_t)(big - 1));
+    if (lane == 0) bits[base >> 5] = word;
+  }
 }
 
 // The vertices outside the giant set, as scan items of their out-buckets
@@ -870,12 +900,18 @@ __global__ void k_uf_compress_ranges(uint32_t *p, const uint32_t *vpre, const ui
 
 // ---- ranges held in shared memory ----
 // A range of at most kUfLocalMax vertices (a member of a graph set) is solved
-// by one CTA with its union-find in shared memory (uf_member).  CTAs take
-// ranges from a counter, largest first.  rng[r] = (first vertex, end vertex,
-// first bucket, end bucket).
+// with its union-find in shared memory (uf_member_link), by one CTA or, when
+// it holds more than one SM's share of all buckets, by several that take a
+// part of its buckets each (uf_member_join).  CTAs take the units from a
+// counter, most buckets first.  rng[r] = (first vertex, end vertex, first
+// bucket, end bucket) of a unit, part[r] = (part, parts, its range's slots /
+// 8, its range's flags).
+// Without the parts one CTA walked the largest member while most SMs were
+// idle: 256 members of 1,024 to 65,535 vertices, 38 M edges, 2.8 ms.
 template <bool kW>
 __global__ void __launch_bounds__(kMemThreads, 1)
-    k_uf_members(GraphView g, const uint4 *__restrict__ rng, uint32_t nr, uint32_t *counter,
+    k_uf_members(GraphView g, const uint4 *__restrict__ rng, const uint4 *__restrict__ part,
+                 uint32_t nr, uint32_t *counter, uint32_t *flags, uint16_t *slots,
                  uint32_t *__restrict__ labels, uint32_t *err) {
   extern __shared__ uint16_t sp[];
   __shared__ uint32_t s_range;
@@ -885,7 +921,11 @@ __global__ void __launch_bounds__(kMemThreads, 1)
     __syncthreads();
     const uint32_t r = s_range;
     if (r >= nr) break;
-    uf_member<kW, false>(g, L, rng[r], labels, err, sp);
+    const uint4 R = rng[r], X = part[r];
+    uf_member_link<kW, false>(g, L, R, err, sp);
+    const uint32_t n = R.y - R.x;
+    if (X.y == 1 || uf_member_join(n, X.x, X.y, (n + 7) & ~7u, slots + (size_t)X.z * 8, flags + X.w, sp, err))
+      uf_member_labels(R, labels, sp);
   }
 }
 
@@ -919,10 +959,13 @@ struct mk_wcc {
   // straight to the static passes: skip_left of them, doubling (to 8) with
   // every further such split, reset by a rescan that succeeds
   uint32_t skip_left = 0, skip_next = 0;
-  // prepared range table: counter word, then uint4 (lo, hi, b0, b1) per small
-  // range (largest first), then vpre, vbase, bpre, bbase of the large ranges
+  // prepared range table: counter word, then the join flags (zeroed with it
+  // before every launch) up to a multiple of 4 words, uint4 (lo, hi, b0, b1)
+  // and uint4 (part, parts, slots / 8, flags) per unit of the small ranges
+  // (most buckets first), then vpre, vbase, bpre, bbase of the large ranges
   DevBuf<uint32_t> ranges;
-  uint32_t n_small = 0, n_large = 0, small_max = 0;
+  DevBuf<uint16_t> slots;  // the parts' sets of the ranges split over several CTAs
+  uint32_t n_units = 0, n_flags = 0, n_large = 0, small_max = 0;
   uint64_t large_vt = 0, large_bt = 0;
   int small_grid = 0;
   bool prepared = false;
@@ -954,12 +997,20 @@ static mk_status wcc_link(mk_wcc *w, const uint32_t *sel, cudaStream_t s) {
   else
     k_uf_sample<false><<<fg, 256, 0, s>>>(v, w->parent, sel, w->err, w->fe);
   k_uf_compress<<<fg, 256, 0, s>>>(w->parent, g->V, sel);
+  uint32_t *big = nullptr;
+  if (!sel) {  // the whole graph: the big set's bits go where the next repair puts its own
+    big = w->aff_vertices;
+    MK_CUDA(cudaMemsetAsync(w->fctl, 0, kFCtlWords * 8, s));
+    k_uf_giant_sample<<<1, kMainThreads, 0, s>>>(w->parent, g->deg, g->V, 0x61A0000ull + (++w->calls),
+                                                 w->fctl);
+    k_uf_big_bits<<<fg, 256, 0, s>>>(w->parent, g->V, w->fctl, big);
+  }
   const int blocks = (int)std::min<uint64_t>(g->num_buckets * 8 / 256 + 1,
                                              (uint64_t)device_sm_count(g->device) * 8);
   if (g->weighted)
-    k_uf_edges_skip<true><<<blocks, 256, 0, s>>>(v, w->parent, sel, w->err, w->fe);
+    k_uf_edges_skip<true><<<blocks, 256, 0, s>>>(v, w->parent, sel, w->err, w->fe, nullptr, big);
   else
-    k_uf_edges_skip<false><<<blocks, 256, 0, s>>>(v, w->parent, sel, w->err, w->fe);
+    k_uf_edges_skip<false><<<blocks, 256, 0, s>>>(v, w->parent, sel, w->err, w->fe, nullptr, big);
   k_uf_compress<<<fg, 256, 0, s>>>(w->parent, g->V, sel);
   MK_CUDA(cudaGetLastError());
   return MK_OK;
@@ -988,6 +1039,8 @@ static mk_status wcc_static(mk_wcc *w, cudaStream_t s) {
   MK_CUDA(cudaMemsetAsync(w->fctl, 0, kFCtlWords * 8, s));
   k_uf_giant_sample<<<1, kMainThreads, 0, s>>>(w->parent, g->deg, V, 0x61A0000ull + (++w->calls),
                                                w->fctl);
+  // (no big-set bits here: with a giant set the pass over every edge returns
+  // at once, and without one they would skip little)
   k_uf_outside_items<<<fg, 256, 0, s>>>(w->parent, V, v, rv, w->fctl, w->items_out.ptr,
                                         w->items_in.ptr);
   const int ob = (int)std::min<uint64_t>(g->num_buckets * 8 / 256 + 1,
@@ -1162,19 +1215,46 @@ static mk_status wcc_prepare(mk_wcc *w, const uint32_t *h_vertex_ranges, uint32_
     (e - b <= kUfLocalMax ? small_ids : large_ids).push_back(r);
   }
   auto len = [&](uint32_t r) { return h_vertex_ranges[2 * r + 1] - h_vertex_ranges[2 * r]; };
-  std::stable_sort(small_ids.begin(), small_ids.end(),
-                   [&](uint32_t a, uint32_t b) { return len(a) > len(b); });
-  const size_t ns = small_ids.size(), nl = large_ids.size();
-  std::vector<uint32_t> host(4 + 4 * ns + 4 * (nl + 1), 0u);
-  uint32_t *sm = host.data() + 4;
-  for (size_t i = 0; i < ns; ++i) {
-    const uint32_t r = small_ids[i], b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
-    sm[4 * i + 0] = b;
-    sm[4 * i + 1] = e;
-    sm[4 * i + 2] = g->h_boff[b];
-    sm[4 * i + 3] = g->h_boff[e];
+  // A small range with more buckets than an SM's share of them all is split
+  // into parts of at most that share (a power of two, at most kMaxParts; a
+  // part under kMinPart buckets costs more to join than it saves).
+  struct Unit {
+    uint32_t r, part, parts, slot, flag, b0, b1;
+  };
+  constexpr uint32_t kMaxParts = 8, kMinPart = 4096;
+  uint64_t all = 0;
+  for (uint32_t r : small_ids) all += g->h_boff[h_vertex_ranges[2 * r + 1]] - g->h_boff[h_vertex_ranges[2 * r]];
+  const uint64_t share = std::max<uint64_t>(all / (uint64_t)device_sm_count(g->device) + 1, kMinPart);
+  std::vector<Unit> units;
+  uint64_t slots8 = 0;  // in units of 8 words
+  uint32_t nflags = 0, smax = 0;
+  for (uint32_t r : small_ids) {
+    const uint32_t b0 = g->h_boff[h_vertex_ranges[2 * r]], b1 = g->h_boff[h_vertex_ranges[2 * r + 1]];
+    uint32_t parts = 1;
+    while (parts < kMaxParts && (uint64_t)parts * share < b1 - b0) parts *= 2;
+    for (uint32_t k = 0; k < parts; ++k)
+      units.push_back({r, k, parts, (uint32_t)slots8, nflags, b0 + (uint32_t)((uint64_t)(b1 - b0) * k / parts),
+                       b0 + (uint32_t)((uint64_t)(b1 - b0) * (k + 1) / parts)});
+    if (parts > 1) {
+      slots8 += (uint64_t)parts * ((len(r) + 7) / 8);
+      nflags += parts;
+    }
+    smax = std::max(smax, len(r));
   }
-  uint32_t *vpre = sm + 4 * ns, *vbase = vpre + nl + 1, *bpre = vbase + nl + 1, *bbase = bpre + nl + 1;
+  std::stable_sort(units.begin(), units.end(),
+                   [](const Unit &a, const Unit &b) { return a.b1 - a.b0 > b.b1 - b.b0; });
+  const size_t nu = units.size(), nl = large_ids.size();
+  const size_t head = (1 + (size_t)nflags + 3) / 4 * 4;
+  std::vector<uint32_t> host(head + 8 * nu + 4 * (nl + 1), 0u);
+  uint32_t *sm = host.data() + head, *pt = sm + 4 * nu;
+  for (size_t i = 0; i < nu; ++i) {
+    const Unit &u = units[i];
+    const uint32_t row[4] = {h_vertex_ranges[2 * u.r], h_vertex_ranges[2 * u.r + 1], u.b0, u.b1};
+    const uint32_t how[4] = {u.part, u.parts, u.slot, u.flag};
+    std::copy(row, row + 4, sm + 4 * i);
+    std::copy(how, how + 4, pt + 4 * i);
+  }
+  uint32_t *vpre = pt + 4 * nu, *vbase = vpre + nl + 1, *bpre = vbase + nl + 1, *bbase = bpre + nl + 1;
   uint64_t vt = 0, bt = 0;
   for (size_t i = 0; i < nl; ++i) {
     const uint32_t r = large_ids[i], b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
@@ -1189,8 +1269,10 @@ static mk_status wcc_prepare(mk_wcc *w, const uint32_t *h_vertex_ranges, uint32_
   bpre[nl] = (uint32_t)bt;
   DeviceGuard dg(g->device);
   w->prepared = false;
-  if (host.size() > w->ranges.cap) MK_CUDA(cudaDeviceSynchronize());  // growth frees the old table
+  if (host.size() > w->ranges.cap || slots8 * 8 > w->slots.cap)
+    MK_CUDA(cudaDeviceSynchronize());  // growth frees the old table
   MK_CHECK(w->ranges.reserve(host.size(), &g->device_bytes));
+  MK_CHECK(w->slots.reserve(std::max<uint64_t>(slots8 * 8, 8), &g->device_bytes));
   if (async) {
     // ordered after the earlier launches on s, which may still read the old table
     MK_CHECK(w->staging.upload(w->ranges.ptr, host.data(), host.size() * 4, s));
@@ -1199,19 +1281,20 @@ static mk_status wcc_prepare(mk_wcc *w, const uint32_t *h_vertex_ranges, uint32_
     MK_CUDA(cudaDeviceSynchronize());
     MK_CUDA(cudaMemcpy(w->ranges.ptr, host.data(), host.size() * 4, cudaMemcpyHostToDevice));
   }
-  w->n_small = (uint32_t)ns;
+  w->n_units = (uint32_t)nu;
+  w->n_flags = nflags;
   w->n_large = (uint32_t)nl;
-  w->small_max = ns ? len(small_ids[0]) : 0;
+  w->small_max = smax;
   w->large_vt = vt;
   w->large_bt = bt;
   w->small_grid = 0;
-  if (ns) {
+  if (nu) {
     const size_t smem = uf_member_smem(w->small_max);
     auto kern = g->weighted ? k_uf_members<true> : k_uf_members<false>;
     MK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)uf_member_smem(kUfLocalMax)));
     int per_sm = 0;
     MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kMemThreads, smem));
-    w->small_grid = (int)std::min<uint64_t>(ns, (uint64_t)device_sm_count(g->device) * std::max(per_sm, 1));
+    w->small_grid = (int)std::min<uint64_t>(nu, (uint64_t)device_sm_count(g->device) * std::max(per_sm, 1));
   }
   w->prepared = true;
   return MK_OK;
@@ -1240,18 +1323,21 @@ mk_status mk_wcc_static_prepared(mk_wcc *w, void *stream, float *ms_out) {
   w->forest_valid = false;  // the range passes record no forest
   const GraphView v = g->view();
   uint32_t *counter = w->ranges.ptr;
-  const uint32_t ns = w->n_small, nl = w->n_large;
-  if (ns) {
+  const uint32_t nu = w->n_units, nl = w->n_large;
+  const size_t head = (1 + (size_t)w->n_flags + 3) / 4 * 4;
+  if (nu) {
     const size_t smem = uf_member_smem(w->small_max);
-    const uint4 *rng = reinterpret_cast<const uint4 *>(w->ranges.ptr + 4);
-    MK_CUDA(cudaMemsetAsync(counter, 0, 4, s));
+    const uint4 *rng = reinterpret_cast<const uint4 *>(w->ranges.ptr + head);
+    MK_CUDA(cudaMemsetAsync(counter, 0, (1 + (size_t)w->n_flags) * 4, s));
     if (g->weighted)
-      k_uf_members<true><<<w->small_grid, kMemThreads, smem, s>>>(v, rng, ns, counter, w->parent, w->err);
+      k_uf_members<true><<<w->small_grid, kMemThreads, smem, s>>>(v, rng, rng + nu, nu, counter, counter + 1,
+                                                                  w->slots.ptr, w->parent, w->err);
     else
-      k_uf_members<false><<<w->small_grid, kMemThreads, smem, s>>>(v, rng, ns, counter, w->parent, w->err);
+      k_uf_members<false><<<w->small_grid, kMemThreads, smem, s>>>(v, rng, rng + nu, nu, counter, counter + 1,
+                                                                   w->slots.ptr, w->parent, w->err);
   }
   if (nl) {
-    const uint32_t *dv = w->ranges.ptr + 4 + 4 * (size_t)ns, *dvb = dv + nl + 1;
+    const uint32_t *dv = w->ranges.ptr + head + 8 * (size_t)nu, *dvb = dv + nl + 1;
     const uint32_t *db = dvb + nl + 1, *dbb = db + nl + 1;
     const int fg = flat_grid(w->large_vt, g->device);
     k_uf_init_ranges<<<fg, 256, 0, s>>>(w->parent, dv, dvb, nl);
@@ -1404,6 +1490,7 @@ mk_status mk_wcc_destroy(mk_wcc *w) {
   w->items_in.release();
   w->staging.release();
   w->ranges.release();
+  w->slots.release();
   delete w;
   return MK_OK;
 }
