@@ -16,10 +16,13 @@
 //   triangle is therefore counted exactly once, at its smallest changed edge.
 //
 // B200 design.  Static: degree-ordered orientation (rank = (deg, id)),
-// oriented CSR built from the slabs (count, scan, fill), then the forward
-// algorithm: a warp stages N+(u) in a shared-memory hash set and streams
-// N+(v) for every v in N+(u) with coalesced 128-byte reads; vertices with a
-// large N+(u) use a block and a global-memory set.  Dynamic: one 8-lane group
+// oriented CSR built from the slabs (count, scan, fill), then every oriented
+// edge {u, v} intersects N+(u) with N+(v): it goes to the endpoint with the
+// longer list (its owner), a warp stages the owner's list in a shared-memory
+// hash set and streams the other endpoints' lists with coalesced reads, so
+// the probes are the sum of the shorter lists (half of streaming N+(v) for
+// every v in N+(u) on R-MAT); owners with a list above kTcSmallMax use a
+// block and a global-memory set.  Dynamic: one 8-lane group
 // per changed edge walks the slabs of the lower-degree endpoint and probes the
 // other endpoint's slab hash per candidate (one lane per candidate).
 #include <cuda_runtime.h>
@@ -159,25 +162,68 @@ __device__ __forceinline__ bool set_contains_cg(const uint32_t *set, uint32_t ca
   return false;
 }
 
-constexpr uint32_t kTcChunk = 32;  // N+(u) entries per work item (one per lane)
+constexpr uint32_t kTcChunk = 64;  // partners per work item
 constexpr int kTcSteps = 4;        // 32-entry probe steps with their loads in flight together
 
-// Work items of the forward algorithm: (u, chunk c) covers N+(u)[32c, 32c+32).
-// Per-vertex work is heavy-tailed (a hub's neighbours have long N+ lists),
-// so vertices are split into chunks and handed out dynamically.  Vertices
-// with N+(u) larger than kTcSmallMax go to the big list instead.
-__global__ void k_tc_item_count(uint32_t V, const unsigned long long *__restrict__ orow,
+// Length of every oriented list.
+__global__ void k_tc_odeg(uint32_t V, const unsigned long long *__restrict__ orow,
+                          uint32_t *__restrict__ odeg) {
+  for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x)
+    odeg[u] = (uint32_t)(orow[u + 1] - orow[u]);
+}
+
+// Partners per owner (kFill false), or the partners written into the owners'
+// rows, the counts used up as cursors (kFill true).  An edge whose shorter
+// list is empty has no triangle and no owner.  An 8-lane group per vertex
+// walks its oriented list; the edges it owns itself take one add per step.
+template <bool kFill>
+__global__ void k_tc_own(uint32_t V, const unsigned long long *__restrict__ orow,
+                         const uint32_t *__restrict__ ocol, const uint32_t *__restrict__ odeg,
+                         uint32_t *__restrict__ pcnt, const unsigned long long *__restrict__ prow,
+                         uint32_t *__restrict__ pcol) {
+  const Lanes L = lanes();
+  const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const uint32_t ngroups = (gridDim.x * blockDim.x) >> 3;
+  for (uint32_t u = group; u < V; u += ngroups) {
+    const uint32_t du = odeg[u];
+    const unsigned long long r0 = orow[u];
+    for (uint32_t j0 = 0; j0 < du; j0 += 8) {
+      const uint32_t j = j0 + L.gl;
+      const uint32_t v = j < du ? ocol[r0 + j] : kEmptyKey;
+      const uint32_t dv = v != kEmptyKey ? odeg[v] : 0u;
+      const bool mine = dv != 0 && du >= dv, theirs = dv > du;
+      const uint32_t mask = __ballot_sync(L.gmask, mine) >> L.gbase;
+      uint32_t at = 0;
+      if (L.gl == 0 && mask)
+        at = kFill ? atomicSub(pcnt + u, (uint32_t)__popc(mask)) : atomicAdd(pcnt + u, (uint32_t)__popc(mask));
+      if (kFill) {
+        at = __shfl_sync(L.gmask, at, L.gbase);
+        if (mine) pcol[prow[u] + (at - 1u - __popc(mask & ((1u << L.gl) - 1u)))] = v;
+        if (theirs) pcol[prow[v] + (atomicSub(pcnt + v, 1u) - 1u)] = u;
+      } else if (theirs) {
+        atomicAdd(pcnt + v, 1u);
+      }
+    }
+  }
+}
+
+// Work items: (h, chunk c) covers partners [64 c, 64 c + 64) of owner h.
+// Per-owner work is heavy-tailed, so owners are split into chunks and handed
+// out dynamically.  Owners whose list is longer than kTcSmallMax go to the
+// big list instead.
+__global__ void k_tc_item_count(uint32_t V, const uint32_t *__restrict__ odeg,
+                                const unsigned long long *__restrict__ prow,
                                 uint32_t *__restrict__ icnt, uint32_t *big_list, uint32_t *big_n,
                                 uint32_t *big_max) {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x) {
-    const uint32_t du = (uint32_t)(orow[u + 1] - orow[u]);
+    const uint32_t du = odeg[u], np = (uint32_t)(prow[u + 1] - prow[u]);
     uint32_t c = 0;
-    if (du >= 2) {  // a triangle needs two oriented edges out of u
+    if (du && np) {
       if (du > kTcSmallMax) {
         big_list[atomicAdd(big_n, 1u)] = u;
         atomicMax(big_max, du);
       } else
-        c = (du + kTcChunk - 1) / kTcChunk;
+        c = (np + kTcChunk - 1) / kTcChunk;
     }
     icnt[u] = c;
   }
@@ -193,19 +239,24 @@ __global__ void k_tc_item_fill(uint32_t V, const uint32_t *__restrict__ icnt,
   }
 }
 
-// Persistent warps take work items from a global counter.  For item (u, c)
-// the warp stages N+(u) in a shared-memory hash set and streams the N+(v)
-// lists of the item's 32 neighbours v as one concatenated range with
-// coalesced reads, probing the set.
+// Persistent warps take work items from a global counter.  For item (h, c)
+// the warp stages N+(h) in a shared-memory hash set and streams the lists of
+// the item's partners one after the other, 32 entries per step and kTcSteps
+// steps of loads in flight: nearly all probes come from lists of more than 64
+// entries, so a list's last, partly empty step costs less than mapping lanes
+// across list ends did (a 5-round shuffle search per step).  The set's first
+// slots are read for all steps before any is compared.  Bound: instruction
+// issue and shared-memory bank conflicts of the probes.
 __global__ void __launch_bounds__(kTcWarps * 32)
     k_tc_small(const unsigned long long *__restrict__ orow, const uint32_t *__restrict__ ocol,
-               const unsigned long long *__restrict__ items, const unsigned long long *nitems_p,
-               uint32_t *next, unsigned long long *count) {
+               const uint32_t *__restrict__ odeg, const unsigned long long *__restrict__ prow,
+               const uint32_t *__restrict__ pcol, const unsigned long long *__restrict__ items,
+               const unsigned long long *nitems_p, uint32_t *next, unsigned long long *count) {
   __shared__ uint32_t sets[kTcWarps][kTcSetCap];
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   uint32_t *set = sets[wib];
   const unsigned long long nitems = *nitems_p;
-  unsigned long long c = 0;
+  unsigned long long total = 0;
   uint32_t have_u = 0xFFFFFFFFu;  // vertex whose set is staged
   uint32_t cap = 64;
   for (;;) {
@@ -215,9 +266,9 @@ __global__ void __launch_bounds__(kTcWarps * 32)
     if (it >= nitems) break;
     const unsigned long long item = items[it];
     const uint32_t u = (uint32_t)item, chunk = (uint32_t)(item >> 32);
-    const unsigned long long r0 = orow[u], r1 = orow[u + 1];
-    const uint32_t du = (uint32_t)(r1 - r0);
     if (u != have_u) {
+      const unsigned long long r0 = orow[u];
+      const uint32_t du = odeg[u];
       __syncwarp();
       // load at most 1/4 (1/2 for the largest sets): most probes miss, and a
       // miss walks the probe run to an EMPTY slot
@@ -229,53 +280,50 @@ __global__ void __launch_bounds__(kTcWarps * 32)
       __syncwarp();
       have_u = u;
     }
-    // the item's (up to 32) neighbours v, one per lane; their N+(v) lists
-    // are walked as one concatenated range, 32 entries per step and
-    // kTcSteps steps of loads in flight, so short lists do not idle lanes
     const uint32_t shift = __clz(cap) + 1;
-    const uint32_t i0 = chunk * kTcChunk, m = min(du, i0 + kTcChunk) - i0;
-    unsigned long long s0 = 0;
-    uint32_t len = 0;
-    if (lane < m) {
-      const uint32_t v = ocol[r0 + i0 + lane];
-      s0 = orow[v];
-      len = (uint32_t)(orow[v + 1] - s0);
-    }
-    uint32_t incl = len;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
-    }
-    const uint32_t off = incl - len;
-    const uint32_t T = __shfl_sync(0xFFFFFFFFu, incl, 31);
-    const unsigned long long basej = s0 - off;  // entry x of lane l's list is ocol[basej(l) + x]
-    for (uint32_t x0 = 0; x0 < T; x0 += 32u * kTcSteps) {
-      uint32_t key[kTcSteps];
-#pragma unroll
-      for (int q = 0; q < kTcSteps; ++q) {
-        const uint32_t x = x0 + 32u * q + lane;
-        uint32_t lo = 0;  // last lane whose list starts at or before x
-#pragma unroll
-        for (int st = 16; st > 0; st >>= 1) {
-          const uint32_t cand = lo + (uint32_t)st;
-          if (__shfl_sync(0xFFFFFFFFu, off, cand) <= x) lo = cand;
-        }
-        const unsigned long long bj = __shfl_sync(0xFFFFFFFFu, basej, lo);
-        key[q] = x < T ? ocol[bj + x] : kEmptyKey;
+    const unsigned long long p0 = prow[u] + (unsigned long long)chunk * kTcChunk;
+    const unsigned long long pe = prow[u + 1];
+    uint32_t c = 0;  // this item's triangles found by the lane (at most 64 lists of 2^32 / 32 entries)
+    for (unsigned long long pb = p0; pb < p0 + kTcChunk && pb < pe; pb += 32) {
+      const uint32_t m = pe - pb < 32 ? (uint32_t)(pe - pb) : 32u;
+      // one partner's list per lane, handed round below
+      unsigned long long ls = 0;
+      uint32_t ll = 0;
+      if (lane < m) {
+        const uint32_t x = pcol[pb + lane];
+        ls = orow[x];
+        ll = odeg[x];
       }
+      for (uint32_t i = 0; i < m; ++i) {
+        const uint32_t *list = ocol + __shfl_sync(0xFFFFFFFFu, ls, i);
+        const uint32_t len = __shfl_sync(0xFFFFFFFFu, ll, i);
+        for (uint32_t x0 = lane; x0 - lane < len; x0 += 32u * kTcSteps) {
+          uint32_t key[kTcSteps], got[kTcSteps];
 #pragma unroll
-      for (int q = 0; q < kTcSteps; ++q)
-        if (key[q] != kEmptyKey) c += set_contains(set, cap - 1, shift, key[q]);
+          for (int q = 0; q < kTcSteps; ++q) key[q] = x0 + 32u * q < len ? __ldg(list + x0 + 32u * q) : kTombKey;
+#pragma unroll
+          for (int q = 0; q < kTcSteps; ++q) got[q] = set[set_slot(key[q], shift)];
+#pragma unroll
+          for (int q = 0; q < kTcSteps; ++q) {
+            // no list holds kTombKey and no set does either
+            if (got[q] == key[q])
+              ++c;
+            else if (got[q] != kEmptyKey && key[q] != kTombKey)
+              c += set_contains(set, cap - 1, shift, key[q]);
+          }
+        }
+      }
     }
+    total += c;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-  if (lane == 0 && c) atomicAdd(count, c);
+  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, o);
+  if (lane == 0 && total) atomicAdd(count, total);
 }
 
 __global__ void k_tc_big(const unsigned long long *__restrict__ orow,
-                         const uint32_t *__restrict__ ocol, const uint32_t *__restrict__ big_list,
+                         const uint32_t *__restrict__ ocol, const unsigned long long *__restrict__ prow,
+                         const uint32_t *__restrict__ pcol, const uint32_t *__restrict__ big_list,
                          const uint32_t *__restrict__ big_n, uint32_t *scratch, uint32_t cap,
                          unsigned long long *count) {
   __shared__ unsigned long long red[32];
@@ -294,8 +342,8 @@ __global__ void k_tc_big(const unsigned long long *__restrict__ orow,
     for (uint32_t i = threadIdx.x; i < du; i += blockDim.x) set_insert(set, cp - 1, shift, ocol[r0 + i]);
     __syncthreads();
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (uint32_t i = warp; i < du; i += nw) {
-      const uint32_t v = ocol[r0 + i];
+    for (unsigned long long i = prow[u] + warp; i < prow[u + 1]; i += nw) {
+      const uint32_t v = pcol[i];
       const unsigned long long s0 = orow[v], s1 = orow[v + 1];
       for (unsigned long long j = s0 + lane; j < s1; j += 32) c += set_contains_cg(set, cp - 1, shift, ocol[j]);
     }
@@ -558,7 +606,17 @@ struct mk_tc {
   uint32_t *small = nullptr;             // [0] big_n
   DevBuf<uint32_t> ocnt, ocol, big_list, big_scratch, bcnt, bfill, bcol, pidx;
   DevBuf<unsigned long long> orow, tmp, brow, pkeys, bpos, items;
+  // list lengths, and the edges by owner (static count)
+  DevBuf<uint32_t> odeg, pcnt, pcol;
+  DevBuf<unsigned long long> prow;
   Timer timer;
+};
+
+// Arrays of the counting pass that hold the list lengths (V words), the
+// edges by owner (a word per oriented edge) and their rows (V + 1).
+struct TcOwners {
+  uint32_t *odeg, *pcnt, *pcol;
+  unsigned long long *prow;
 };
 
 struct mk_tc_range {
@@ -574,7 +632,7 @@ static int groups_grid(uint64_t items, int device) {
   return (int)std::min(b, cap);
 }
 
-static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, cudaStream_t s);
+static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, TcOwners own, cudaStream_t s);
 
 static mk_status tc_static(mk_tc *t, cudaStream_t s) {
   mk_graph *g = t->g;
@@ -601,14 +659,38 @@ static mk_status tc_static(mk_tc *t, cudaStream_t s) {
   else
     k_orient_fill<false><<<blocks, 256, 0, s>>>(gv, t->bpos.ptr, t->ocol.ptr);
   MK_CUDA(cudaGetLastError());
-  return tc_count_oriented(t, V, g->device, s);
+  MK_CHECK(t->odeg.reserve(V, &acc));
+  TcOwners own{t->odeg.ptr, nullptr, nullptr, nullptr};
+  // without room for the edges by owner, every edge stays with its lower end
+  if (t->pcol.reserve(std::max<unsigned long long>(total, 1), &acc) == MK_OK &&
+      t->prow.reserve((size_t)V + 1, &acc) == MK_OK && t->pcnt.reserve(V, &acc) == MK_OK)
+    own = {t->odeg.ptr, t->pcnt.ptr, t->pcol.ptr, t->prow.ptr};
+  else
+    (void)cudaGetLastError();
+  return tc_count_oriented(t, V, g->device, own, s);
 }
 
-// The forward algorithm on the oriented CSR in t->orow / t->ocol over V
-// vertices; the count lands in t->dcount[0].  t->ocnt (>= V words) and
-// t->bpos (>= V + 1) serve as scratch.
-static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, cudaStream_t s) {
+// The intersections over the oriented CSR in t->orow / t->ocol, V vertices;
+// the count lands in t->dcount[0].  t->ocnt (>= V words) and t->bpos
+// (>= V + 1) serve as scratch.  own.pcol null: the edges stay with their
+// lower ends (the oriented CSR itself).
+static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, TcOwners own, cudaStream_t s) {
   size_t acc = 0;
+  const unsigned long long *prow = t->orow.ptr;
+  const uint32_t *pcol = t->ocol.ptr;
+  {
+    const int vb = (int)std::min<uint64_t>((uint64_t)V / 256 + 1, (uint64_t)device_sm_count(device) * 8);
+    k_tc_odeg<<<vb, 256, 0, s>>>(V, t->orow.ptr, own.odeg);
+    if (own.pcol) {
+      const int gb = groups_grid(V, device);
+      MK_CUDA(cudaMemsetAsync(own.pcnt, 0, (size_t)V * 4, s));
+      k_tc_own<false><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, nullptr, nullptr);
+      MK_CHECK(scan_u32_to_u64(own.pcnt, own.prow, V, t->tmp, s));
+      k_tc_own<true><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, own.prow, own.pcol);
+      prow = own.prow;
+      pcol = own.pcol;
+    }
+  }
   MK_CHECK(t->big_list.reserve(V, &acc));
   MK_CUDA(cudaMemsetAsync(t->dcount, 0, 8, s));
   // [0] big count, [1] work-item counter, [2] largest big oriented degree
@@ -616,7 +698,7 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, cudaStream_
   // work items (the orientation scratch is free again: ocnt >= V words,
   // bpos >= V + 1)
   const int vb = (int)std::min<uint64_t>((uint64_t)V / 256 + 1, (uint64_t)device_sm_count(device) * 8);
-  k_tc_item_count<<<vb, 256, 0, s>>>(V, t->orow.ptr, t->ocnt.ptr, t->big_list.ptr, t->small,
+  k_tc_item_count<<<vb, 256, 0, s>>>(V, own.odeg, prow, t->ocnt.ptr, t->big_list.ptr, t->small,
                                      t->small + 2);
   MK_CHECK(scan_u32_to_u64(t->ocnt.ptr, t->bpos.ptr, V, t->tmp, s));
   unsigned long long nitems = 0;
@@ -629,7 +711,7 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, cudaStream_
   int per_sm = 0;
   MK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tc_small, kTcWarps * 32, 0));
   const int sblocks = device_sm_count(device) * std::max(per_sm, 1);
-  k_tc_small<<<sblocks, kTcWarps * 32, 0, s>>>(t->orow.ptr, t->ocol.ptr, t->items.ptr,
+  k_tc_small<<<sblocks, kTcWarps * 32, 0, s>>>(t->orow.ptr, t->ocol.ptr, own.odeg, prow, pcol, t->items.ptr,
                                               t->bpos.ptr + V, t->small + 1, t->dcount);
   // big vertices: one block each, global-memory set
   const uint32_t nbig = hs[0];
@@ -640,7 +722,7 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, cudaStream_
     while (cap < 2ull * mx) cap <<= 1;
     int bb = std::min<uint32_t>(nbig, (uint32_t)device_sm_count(device) * 2);
     MK_CHECK(t->big_scratch.reserve((size_t)bb * cap, &acc));
-    k_tc_big<<<bb, 512, 0, s>>>(t->orow.ptr, t->ocol.ptr, t->big_list.ptr, t->small,
+    k_tc_big<<<bb, 512, 0, s>>>(t->orow.ptr, t->ocol.ptr, prow, pcol, t->big_list.ptr, t->small,
                                 t->big_scratch.ptr, cap, t->dcount);
   }
   MK_CUDA(cudaGetLastError());
@@ -817,7 +899,10 @@ mk_status mk_tc_range_run(mk_tc_range *t, uint32_t v_begin, uint32_t v_end, void
   k_trc_orient<true><<<eb, 256, 0, s>>>(t->rowid.ptr, t->col.ptr, lo, E, t->rflag.ptr,
                                         t->dsym.ptr, c->ocnt.ptr, c->orow.ptr, c->ocol.ptr);
   MK_CUDA(cudaGetLastError());
-  MK_CHECK(tc_count_oriented(c, n, g->device, s));
+  // the member's CSR rows, row ids and degree counts are done with: they hold
+  // the edges by owner
+  const TcOwners own{t->recip.ptr, t->indeg.ptr, t->rowid.ptr, t->rp.ptr};
+  MK_CHECK(tc_count_oriented(c, n, g->device, own, s));
   return c->timer.stop(ms_out);
 }
 
@@ -872,6 +957,10 @@ mk_status mk_tc_destroy(mk_tc *t) {
   t->bfill.release();
   t->bcol.release();
   t->pidx.release();
+  t->odeg.release();
+  t->pcnt.release();
+  t->pcol.release();
+  t->prow.release();
   t->orow.release();
   t->tmp.release();
   t->brow.release();

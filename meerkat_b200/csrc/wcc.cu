@@ -289,7 +289,7 @@ __global__ void k_uf_edges_skip(GraphView g, uint32_t *p, const uint32_t *sel_bi
       uint32_t pj = pu[0] * (j == 0) + pu[1] * (j == 1) + pu[2] * (j == 2) + pu[3] * (j == 3);
       uint32_t k[4], w[4];
       lane_keys<kW>(q, L.gl, k, w);
-      uint32_t pv[4];
+      uint32_t pv[4] = {0u, 0u, 0u, 0u};
       bool ok[4];
 #pragma unroll
       for (int t = 0; t < keys_per_lane<kW>(); ++t) {
@@ -301,9 +301,14 @@ __global__ void k_uf_edges_skip(GraphView g, uint32_t *p, const uint32_t *sel_bi
         ok[t] = ok[t] && !((pv[t] >> (k[t] & 31)) & 1u);
         pv[t] = ok[t] ? __ldcg(p + k[t]) : 0u;
       }
+      uint32_t need = 0;
 #pragma unroll
-      for (int t = 0; t < keys_per_lane<kW>(); ++t)
-        if (ok[t] && pv[t] != pj) pj = uf_union_root(p, u, k[t], err, fe);
+      for (int t = 0; t < keys_per_lane<kW>(); ++t) need |= (ok[t] && pv[t] != pj ? 1u : 0u) << t;
+      for (; need; need &= need - 1) {  // one call site: the walk copies this body eight times
+        const uint32_t kt = need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3];
+        const uint32_t pt = need & 1u ? pv[0] : need & 2u ? pv[1] : need & 4u ? pv[2] : pv[3];
+        if (pt != pj) pj = uf_union_root(p, u, kt, err, fe);
+      }
 #pragma unroll
       for (uint32_t i = 0; i < 4; ++i)
         if (i == j) pu[i] = pj;
