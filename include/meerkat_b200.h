@@ -193,8 +193,9 @@ typedef struct mk_tuning {
                                     1..1024, 0 = 4                            */
   uint32_t sssp_delta;           /* static SSSP near-far step: relaxations to
                                     distances >= threshold wait on a far list
-                                    until the near frontier drains; 0 = off
-                                    (plain level-synchronous)                  */
+                                    until the near frontier drains, then the
+                                    threshold moves on by this much; 0 =
+                                    automatic (it doubles)                     */
   uint32_t recompute_permille;   /* decremental BFS/SSSP: once this share of
                                     the vertices (per mille) is invalidated,
                                     recompute from the sources instead of
@@ -270,12 +271,14 @@ mk_status mk_traversal_static(mk_traversal *t, void *stream, float *ms_out);
  * (blocking; it waits for the device, since queued work may read the
  * previous table); static_members runs it and issues only asynchronous work
  * on `stream`, so it can be captured into a CUDA graph.  A range of at most
- * 65,535 vertices is solved by one CTA with its BFS state in shared memory;
+ * 65,535 vertices is solved by one CTA with its BFS state in shared memory,
+ * unless it holds more than two SMs' share of all ranges' buckets; such and
  * larger ones by the device-wide kernel.  The distances of every vertex are
  * those mk_traversal_static gives and the parents form a valid BFS tree
  * (parents are not unique: of several equal-distance parents, the device-wide
  * kernel keeps the first to arrive, the member kernel the smallest id); an
- * edge leaving its range sets MK_DEVERR_INVALID_ID on the graph.  BFS only.
+ * edge leaving a range of at most 65,535 vertices sets MK_DEVERR_INVALID_ID on
+ * the graph.  BFS only.
  * No counterpart in the reference. */
 mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_ranges,
                                  uint32_t nranges);

@@ -256,8 +256,8 @@ mk_status mk_set_runner_create(mk_graphset *s, const uint8_t *h_query,
     if (st == MK_OK) st = mk_wcc_prepare_ranges(r->wcc, wcc_ranges.data(), r->n_wcc);
   }
   if (st == MK_OK && r->bfs && r->wcc && max_member <= kMemLocalMax) {
-    // (larger members go through device-wide kernels, one of them a
-    // cooperative launch that needs every SM: no room beside it)
+    // (larger members take the components through device-wide kernels too:
+    // those run in order)
     DeviceGuard dg(g->device);
     cudaError_t e = cudaStreamCreateWithFlags(&r->side, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
@@ -286,7 +286,7 @@ mk_status mk_set_runner_set_single(mk_set_runner *r, uint32_t on) {
 
 mk_status mk_set_runner_launches(mk_set_runner *r, uint32_t *h_launches) {
   if (!r || !h_launches) return fail(MK_ERR_INVALID, "mk_set_runner_launches: null argument");
-  *h_launches = r->single ? 1u : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u);
+  *h_launches = r->single ? 1u : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u) + (trav_members_wide(r->bfs) ? 1u : 0u);
   return MK_OK;
 }
 
@@ -347,17 +347,18 @@ mk_status mk_set_runner_step(mk_set_runner *r, const uint32_t *d_del_src,
   if (r->side) {
     // Both query kernels end in a tail of few busy SMs (a member per CTA, an
     // eightfold spread of sizes); side by side each fills the other's.  They
-    // share only the graph, which neither writes.
+    // share only the graph, which neither writes.  The fork stands behind the
+    // BFS's device-wide part, a cooperative launch that needs every SM.
     DeviceGuard dg(r->g->device);
     cudaStream_t s = as_stream(stream);
-    MK_CUDA(cudaEventRecord(r->fork, s));
+    const mk_status bs = trav_static_members(r->bfs, stream, nullptr, r->fork);
+    if (bs != MK_OK) return bs;  // nothing forked that is not joined
     MK_CUDA(cudaStreamWaitEvent(r->side, r->fork, 0));
-    const mk_status bs = mk_bfs_static_members(r->bfs, stream, nullptr);
     const mk_status ws = mk_wcc_static_prepared(r->wcc, r->side, nullptr);
     // joined whatever happened: the caller's stream stays ordered behind both
     MK_CUDA(cudaEventRecord(r->join, r->side));
     MK_CUDA(cudaStreamWaitEvent(s, r->join, 0));
-    return bs != MK_OK ? bs : ws;
+    return ws;
   }
   if (r->bfs) MK_CHECK(mk_bfs_static_members(r->bfs, stream, nullptr));
   if (r->wcc) MK_CHECK(mk_wcc_static_prepared(r->wcc, stream, nullptr));

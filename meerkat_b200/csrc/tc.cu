@@ -117,8 +117,7 @@ constexpr int kTcWarps = 4;           // warps per block in the small kernel (32
 constexpr int kTcSetCap = 2048;       // per-warp shared hash capacity (entries)
 constexpr uint32_t kTcSmallMax = 1024;  // N+(u) handled by one warp
 
-// Open-addressing sets of capacity 2^k (k >= 6), at most half full (a
-// quarter where the warp's share of shared memory allows), with
+// Open-addressing sets of capacity 2^k (k >= 6), at most half full, with
 // Fibonacci hashing: the slot is the top k bits of key * 2654435769 (one
 // multiply and one shift per probe; the sets are probed far more often than
 // built).  shift = 32 - k.  Probes are bounded by the capacity.
@@ -136,20 +135,8 @@ __device__ __forceinline__ void set_insert(uint32_t *set, uint32_t cap_mask, uin
   }
 }
 
-__device__ __forceinline__ bool set_contains(const uint32_t *set, uint32_t cap_mask, uint32_t shift,
-                                             uint32_t key) {
-  uint32_t h = set_slot(key, shift);
-  for (uint32_t it = 0; it <= cap_mask; ++it) {
-    uint32_t k = set[h];
-    if (k == key) return true;
-    if (k == kEmptyKey) return false;
-    h = (h + 1) & cap_mask;
-  }
-  return false;
-}
-
-// Same probe for a set in global memory, read through L2 (the set is
-// rebuilt for every vertex, so L1 may hold stale lines).
+// Probe of a set in global memory, read through L2 (the set is rebuilt for
+// every vertex, so L1 may hold stale lines).
 __device__ __forceinline__ bool set_contains_cg(const uint32_t *set, uint32_t cap_mask,
                                                 uint32_t shift, uint32_t key) {
   uint32_t h = set_slot(key, shift);
@@ -160,6 +147,38 @@ __device__ __forceinline__ bool set_contains_cg(const uint32_t *set, uint32_t ca
     h = (h + 1) & cap_mask;
   }
   return false;
+}
+
+// A warp's set in shared memory: buckets of 4 slots filled in order, so one
+// 16-byte read answers a probe unless the bucket is full without the key
+// (then the next bucket is read).  nb buckets, a power of two.  A set of
+// single slots needed a second look on a quarter of the probes, and one such
+// lane holds its whole warp.
+__device__ __forceinline__ uint32_t bucket_slot(uint32_t key, uint32_t bshift) {
+  return (key * 2654435769u) >> bshift;
+}
+
+__device__ __forceinline__ void bucket_insert(uint4 *set, uint32_t nb, uint32_t bshift, uint32_t key) {
+  uint32_t h = bucket_slot(key, bshift);
+  for (uint32_t it = 0; it < nb; ++it) {
+    uint32_t *w = reinterpret_cast<uint32_t *>(set + h);
+    for (int s = 0; s < 4; ++s) {
+      const uint32_t old = atomicCAS(w + s, kEmptyKey, key);
+      if (old == kEmptyKey || old == key) return;
+    }
+    h = (h + 1) & (nb - 1);
+  }
+}
+
+// The rest of a probe whose bucket h was full without the key.
+__device__ __noinline__ uint32_t bucket_probe_on(const uint4 *set, uint32_t nb, uint32_t h, uint32_t key) {
+  for (uint32_t it = 1; it < nb; ++it) {
+    h = (h + 1) & (nb - 1);
+    const uint4 b = set[h];
+    if (b.x == key || b.y == key || b.z == key || b.w == key) return 1u;
+    if (b.w == kEmptyKey) return 0u;
+  }
+  return 0u;
 }
 
 constexpr uint32_t kTcChunk = 64;  // partners per work item
@@ -187,21 +206,39 @@ __global__ void k_tc_own(uint32_t V, const unsigned long long *__restrict__ orow
   for (uint32_t u = group; u < V; u += ngroups) {
     const uint32_t du = odeg[u];
     const unsigned long long r0 = orow[u];
-    for (uint32_t j0 = 0; j0 < du; j0 += 8) {
-      const uint32_t j = j0 + L.gl;
-      const uint32_t v = j < du ? ocol[r0 + j] : kEmptyKey;
-      const uint32_t dv = v != kEmptyKey ? odeg[v] : 0u;
-      const bool mine = dv != 0 && du >= dv, theirs = dv > du;
-      const uint32_t mask = __ballot_sync(L.gmask, mine) >> L.gbase;
+    // four steps of loads in flight: the longest lists are the tail
+    for (uint32_t j0 = 0; j0 < du; j0 += 32) {
+      uint32_t v[4], dv[4], mask[4], total = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t j = j0 + 8u * q + L.gl;
+        v[q] = j < du ? ocol[r0 + j] : kEmptyKey;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) dv[q] = v[q] != kEmptyKey ? odeg[v[q]] : 0u;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        mask[q] = __ballot_sync(L.gmask, dv[q] != 0 && du >= dv[q]) >> L.gbase;
+        total += __popc(mask[q]);
+      }
       uint32_t at = 0;
-      if (L.gl == 0 && mask)
-        at = kFill ? atomicSub(pcnt + u, (uint32_t)__popc(mask)) : atomicAdd(pcnt + u, (uint32_t)__popc(mask));
+      if (L.gl == 0 && total) at = kFill ? atomicSub(pcnt + u, total) : atomicAdd(pcnt + u, total);
       if (kFill) {
+        uint32_t left[4];  // entries still free in the other owners' rows
+#pragma unroll
+        for (int q = 0; q < 4; ++q) left[q] = dv[q] > du ? atomicSub(pcnt + v[q], 1u) : 0u;
         at = __shfl_sync(L.gmask, at, L.gbase);
-        if (mine) pcol[prow[u] + (at - 1u - __popc(mask & ((1u << L.gl) - 1u)))] = v;
-        if (theirs) pcol[prow[v] + (atomicSub(pcnt + v, 1u) - 1u)] = u;
-      } else if (theirs) {
-        atomicAdd(pcnt + v, 1u);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          if ((mask[q] >> L.gl) & 1u)
+            pcol[prow[u] + (at - 1u - __popc(mask[q] & ((1u << L.gl) - 1u)))] = v[q];
+          at -= __popc(mask[q]);
+          if (left[q]) pcol[prow[v[q]] + (left[q] - 1u)] = u;
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (dv[q] > du) atomicAdd(pcnt + v[q], 1u);
       }
     }
   }
@@ -244,21 +281,20 @@ __global__ void k_tc_item_fill(uint32_t V, const uint32_t *__restrict__ icnt,
 // the item's partners one after the other, 32 entries per step and kTcSteps
 // steps of loads in flight: nearly all probes come from lists of more than 64
 // entries, so a list's last, partly empty step costs less than mapping lanes
-// across list ends did (a 5-round shuffle search per step).  The set's first
-// slots are read for all steps before any is compared.  Bound: instruction
-// issue and shared-memory bank conflicts of the probes.
+// across list ends did (a 5-round shuffle search per step).  Bound: bank
+// conflicts of the probes' 16-byte reads, then instruction issue.
 __global__ void __launch_bounds__(kTcWarps * 32)
     k_tc_small(const unsigned long long *__restrict__ orow, const uint32_t *__restrict__ ocol,
                const uint32_t *__restrict__ odeg, const unsigned long long *__restrict__ prow,
                const uint32_t *__restrict__ pcol, const unsigned long long *__restrict__ items,
                const unsigned long long *nitems_p, uint32_t *next, unsigned long long *count) {
-  __shared__ uint32_t sets[kTcWarps][kTcSetCap];
+  __shared__ uint4 sets[kTcWarps][kTcSetCap / 4];
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  uint32_t *set = sets[wib];
+  uint4 *set = sets[wib];
   const unsigned long long nitems = *nitems_p;
   unsigned long long total = 0;
   uint32_t have_u = 0xFFFFFFFFu;  // vertex whose set is staged
-  uint32_t cap = 64;
+  uint32_t nb = 16, bshift = 28;  // its buckets
   for (;;) {
     uint32_t it = 0;
     if (lane == 0) it = atomicAdd(next, 1u);
@@ -270,17 +306,17 @@ __global__ void __launch_bounds__(kTcWarps * 32)
       const unsigned long long r0 = orow[u];
       const uint32_t du = odeg[u];
       __syncwarp();
-      // load at most 1/4 (1/2 for the largest sets): most probes miss, and a
-      // miss walks the probe run to an EMPTY slot
-      cap = 64;
-      while (cap < 4 * du && cap < (uint32_t)kTcSetCap) cap <<= 1;
-      for (uint32_t i = lane; i < cap; i += 32) set[i] = kEmptyKey;
+      // half a key per bucket (two for the largest sets): a bucket is then
+      // full once in 500 probes
+      nb = 16;
+      while (nb < 2 * du && nb < (uint32_t)kTcSetCap / 4) nb <<= 1;
+      bshift = __clz(nb) + 1;
+      for (uint32_t i = lane; i < nb; i += 32) set[i] = make_uint4(kEmptyKey, kEmptyKey, kEmptyKey, kEmptyKey);
       __syncwarp();
-      for (uint32_t i = lane; i < du; i += 32) set_insert(set, cap - 1, __clz(cap) + 1, ocol[r0 + i]);
+      for (uint32_t i = lane; i < du; i += 32) bucket_insert(set, nb, bshift, ocol[r0 + i]);
       __syncwarp();
       have_u = u;
     }
-    const uint32_t shift = __clz(cap) + 1;
     const unsigned long long p0 = prow[u] + (unsigned long long)chunk * kTcChunk;
     const unsigned long long pe = prow[u + 1];
     uint32_t c = 0;  // this item's triangles found by the lane (at most 64 lists of 2^32 / 32 entries)
@@ -298,18 +334,18 @@ __global__ void __launch_bounds__(kTcWarps * 32)
         const uint32_t *list = ocol + __shfl_sync(0xFFFFFFFFu, ls, i);
         const uint32_t len = __shfl_sync(0xFFFFFFFFu, ll, i);
         for (uint32_t x0 = lane; x0 - lane < len; x0 += 32u * kTcSteps) {
-          uint32_t key[kTcSteps], got[kTcSteps];
+          uint32_t key[kTcSteps];
+          // past the end: kTombKey, which no list and no set holds
 #pragma unroll
           for (int q = 0; q < kTcSteps; ++q) key[q] = x0 + 32u * q < len ? __ldg(list + x0 + 32u * q) : kTombKey;
 #pragma unroll
-          for (int q = 0; q < kTcSteps; ++q) got[q] = set[set_slot(key[q], shift)];
-#pragma unroll
           for (int q = 0; q < kTcSteps; ++q) {
-            // no list holds kTombKey and no set does either
-            if (got[q] == key[q])
+            const uint32_t h = bucket_slot(key[q], bshift);
+            const uint4 w = set[h];
+            if (w.x == key[q] || w.y == key[q] || w.z == key[q] || w.w == key[q])
               ++c;
-            else if (got[q] != kEmptyKey && key[q] != kTombKey)
-              c += set_contains(set, cap - 1, shift, key[q]);
+            else if (w.w != kEmptyKey && key[q] != kTombKey)
+              c += bucket_probe_on(set, nb, h, key[q]);
           }
         }
       }

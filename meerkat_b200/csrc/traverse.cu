@@ -91,6 +91,11 @@ struct TravArgs {
   uint32_t bn;
   const uint32_t *sources;  // distinct source vertices (one per query)
   uint32_t nsources;
+  // static BFS of graph-set members: the ranges [x, y), in increasing order,
+  // whose edges must not leave them (an edge that does is skipped and
+  // reported as MK_DEVERR_INVALID_ID, as the member kernel does)
+  const uint2 *closed;
+  uint32_t nclosed;
   uint32_t chunk;           // buckets per frontier work item
   uint32_t mode;
   uint32_t delta;           // near-far SSSP step (0: the threshold doubles)
@@ -117,6 +122,7 @@ constexpr uint32_t kWarpQueue = 192;   // vertices a warp's queue holds
 constexpr uint32_t kWarpFlush = 96;    // vertices from which it is emptied between two rounds
 constexpr uint32_t kFarQueue = 160;    // the same for the far list (SSSP)
 constexpr uint32_t kFarFlush = 80;
+constexpr uint32_t kHeavyBuckets = 32768;  // a member below this never goes device-wide for its buckets
 constexpr uint32_t kDefaultChunk = 4;  // buckets per frontier work item
 
 __host__ __device__ __forceinline__ unsigned long long item(uint32_t v, uint32_t chunk) {
@@ -406,15 +412,20 @@ __device__ __forceinline__ void expand_range(const TravArgs &a, const Lanes &L, 
 template <bool kW>
 __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, const WarpQueue &Q,
                                              const uint4 (&q)[4], uint32_t nq, uint32_t u,
-                                             uint32_t lvl, unsigned long long *gfr, uint32_t *gsz) {
+                                             uint32_t lo, uint32_t span, uint32_t lvl,
+                                             unsigned long long *gfr, uint32_t *gsz) {
   constexpr int KP = keys_per_lane<kW>();
   uint32_t k[4][4], w[4][4], bits[4][KP];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     lane_keys<kW>(q[j], L.gl, k[j], w[j]);
 #pragma unroll
-    for (int i = 0; i < KP; ++i)
-      bits[j][i] = ((uint32_t)j < nq && k[j][i] < kTombKey) ? __ldca(a.vis + (k[j][i] >> 5)) : ~0u;
+    for (int i = 0; i < KP; ++i) {
+      const bool live = (uint32_t)j < nq && k[j][i] < kTombKey;
+      const bool in = k[j][i] - lo < span;
+      if (live && !in) atomicOr(a.g.err, kErrInvalidId);
+      bits[j][i] = live && in ? __ldca(a.vis + (k[j][i] >> 5)) : ~0u;
+    }
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
@@ -427,6 +438,27 @@ __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, 
       if (atomicOr(word, m) & m) continue;
       a.dist[v] = pack(lvl + 1, u);
       push_vertex(a, Q, v, gfr, gsz);
+    }
+  }
+}
+
+// The closed range of TravArgs that holds u, as its first vertex and size
+// (everything when none does).
+__device__ __forceinline__ void closed_range(const TravArgs &a, uint32_t u, uint32_t &lo, uint32_t &span) {
+  lo = 0u;
+  span = kTombKey;
+  uint32_t l = 0, h = a.nclosed;
+  while (l < h) {
+    const uint32_t m = (l + h) >> 1;
+    const uint2 r = __ldg(a.closed + m);
+    if (u < r.x) {
+      h = m;
+    } else if (u >= r.y) {
+      l = m + 1;
+    } else {
+      lo = r.x;
+      span = r.y - r.x;
+      return;
     }
   }
 }
@@ -957,8 +989,10 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
           uint32_t u, b0, b1;
           item_range(a.g, now, a.chunk, u, b0, b1);
           if (!kUseW && a.vis) {
+            uint32_t lo, span;
+            closed_range(a, u, lo, span);
             expand_range(a, L, b0, b1, [&](const uint4 (&q)[4], uint32_t nq) {
-              visit_slabs4<kW>(a, L, Q, q, nq, u, lv, nxt, nsz);
+              visit_slabs4<kW>(a, L, Q, q, nq, u, lo, span, lv, nxt, nsz);
             });
           } else {
             unsigned long long pu = 0;
@@ -1082,6 +1116,8 @@ struct mk_traversal {
   // range is too large for shared memory
   DevBuf<uint32_t> members;
   uint32_t n_small = 0, n_large = 0, small_max = 0;
+  const uint2 *d_closed = nullptr;  // in members: the ranges that went device-wide for their buckets
+  uint32_t n_closed = 0;
   int small_grid = 0;
   bool members_prepared = false;
   PinnedRing staging;  // stream-ordered source uploads
@@ -1251,6 +1287,8 @@ static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, 
   a.bn = n;
   a.sources = srcs ? srcs : t->sources;
   a.nsources = srcs ? nsrc : t->nsources;
+  a.closed = srcs ? t->d_closed : nullptr;
+  a.nclosed = srcs ? t->n_closed : 0u;
   a.chunk = g->tuning.frontier_chunk ? g->tuning.frontier_chunk : kDefaultChunk;
   a.delta = g->tuning.sssp_delta;
   a.rg = t->rev ? t->rev->view() : GraphView{};
@@ -1306,6 +1344,8 @@ static mk_status trav_launch(mk_traversal *t, uint32_t mode, const uint32_t *bs,
 }
 
 namespace mk {
+bool trav_members_wide(const mk_traversal *t) { return t && t->n_large != 0; }
+
 mk_status trav_member_bufs(mk_traversal *t, TravMemberBufs *out) {
   if (!t || !out) return fail(MK_ERR_INVALID, "trav_member_bufs: null argument");
   out->dist = t->dist;
@@ -1439,17 +1479,32 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   mk_graph *g = t->g;
   std::vector<uint32_t> small_ids, large_src;
   std::vector<std::pair<uint32_t, uint32_t>> spans;
+  std::vector<std::pair<uint32_t, uint32_t>> closed;  // small enough, but heavy
+  uint64_t all = 0;  // buckets of all ranges
   for (uint32_t r = 0; r < nranges; ++r) {
     const uint32_t b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
     if (b >= e || e > g->V) return fail(MK_ERR_INVALID, std::string(what) + ": bad vertex range");
     if (t->h_sources[r] < b || t->h_sources[r] >= e)
       return fail(MK_ERR_INVALID, std::string(what) + ": source outside its range");
     spans.emplace_back(b, e);
-    if (e - b <= kMemLocalMax)
-      small_ids.push_back(r);
-    else
-      large_src.push_back(t->h_sources[r]);
+    all += g->h_boff[e] - g->h_boff[b];
   }
+  // A range goes to the device-wide kernel when it is too large for shared
+  // memory, or holds more than twice an SM's share of all buckets (and
+  // enough of them to fill the device): its one CTA would still be walking it
+  // when the other SMs are done.  Of 256 members of 1,024 to 65,535 vertices
+  // (19 M edges) the largest held 8 shares and took the whole 2.3 ms.
+  const uint64_t heavy = std::max<uint64_t>(2 * all / (uint64_t)device_sm_count(g->device), kHeavyBuckets);
+  for (uint32_t r = 0; r < nranges; ++r) {
+    const uint32_t b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
+    if (e - b <= kMemLocalMax && g->h_boff[e] - g->h_boff[b] <= heavy) {
+      small_ids.push_back(r);
+    } else {
+      large_src.push_back(t->h_sources[r]);
+      if (e - b <= kMemLocalMax) closed.emplace_back(b, e);
+    }
+  }
+  std::sort(closed.begin(), closed.end());
   std::sort(spans.begin(), spans.end());
   for (size_t i = 1; i < spans.size(); ++i)
     if (spans[i].first < spans[i - 1].second)
@@ -1463,8 +1518,14 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   std::stable_sort(small_ids.begin(), small_ids.end(),
                    [&](uint32_t a, uint32_t b) { return buckets(a) > buckets(b); });
   const size_t ns = small_ids.size(), nl = large_src.size();
-  std::vector<uint32_t> host(4 + 5 * ns + nl, 0u);
+  const size_t nc = closed.size();
+  const size_t lists = (4 + 5 * ns + nl + 1) / 2 * 2;  // the pairs behind start on 8 bytes
+  std::vector<uint32_t> host(lists + 2 * nc, 0u);
   uint32_t *tab = host.data() + 4, *ssrc = tab + 4 * ns, *lsrc = ssrc + ns;
+  for (size_t i = 0; i < nc; ++i) {
+    host[lists + 2 * i] = closed[i].first;
+    host[lists + 2 * i + 1] = closed[i].second;
+  }
   for (size_t i = 0; i < ns; ++i) {
     const uint32_t r = small_ids[i], b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
     tab[4 * i + 0] = b;
@@ -1482,6 +1543,8 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   MK_CUDA(cudaMemcpy(t->members.ptr, host.data(), host.size() * 4, cudaMemcpyHostToDevice));
   t->n_small = (uint32_t)ns;
   t->n_large = (uint32_t)nl;
+  t->n_closed = (uint32_t)nc;
+  t->d_closed = reinterpret_cast<const uint2 *>(t->members.ptr + lists);
   t->small_max = 0;
   for (uint32_t r : small_ids) t->small_max = std::max(t->small_max, len(r));
   t->small_grid = 0;
@@ -1499,6 +1562,13 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
 }
 
 mk_status mk_bfs_static_members(mk_traversal *t, void *stream, float *ms_out) {
+  return trav_static_members(t, stream, ms_out, nullptr);
+}
+
+}  // extern "C"
+
+namespace mk {
+mk_status trav_static_members(mk_traversal *t, void *stream, float *ms_out, cudaEvent_t wide_done) {
   if (!t) return fail(MK_ERR_INVALID, "mk_bfs_static_members: null handle");
   if (!t->members_prepared) return fail(MK_ERR_INVALID, "mk_bfs_static_members: no prepared ranges");
   mk_graph *g = t->g;
@@ -1516,6 +1586,7 @@ mk_status mk_bfs_static_members(mk_traversal *t, void *stream, float *ms_out) {
   } else {
     trav_begin(t, true, false, false, s);
   }
+  if (wide_done) MK_CUDA(cudaEventRecord(wide_done, s));
   if (ns) {
     const size_t smem = bfs_member_smem(t->small_max);
     MK_CUDA(cudaMemsetAsync(counter, 0, 4, s));
@@ -1532,6 +1603,9 @@ mk_status mk_bfs_static_members(mk_traversal *t, void *stream, float *ms_out) {
   t->has_static = true;
   return MK_OK;
 }
+}  // namespace mk
+
+extern "C" {
 
 mk_status mk_traversal_incremental(mk_traversal *t, const uint32_t *d_src,
                                    const uint32_t *d_dst, const uint32_t *d_w,

@@ -51,3 +51,38 @@ def test_wcc_of_members_split_into_parts(kind, weighted):
             O.insert(ms, md)
             np.testing.assert_array_equal(lab[off[i]:off[i + 1]] - off[i], O.wcc())
     assert gs.graph.sync() == 0
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_bfs_of_members_that_outweigh_the_others(weighted):
+    """One member holds most buckets, so it goes through the device-wide
+    kernel beside the others' shared-memory one; levels are each member's
+    own, and an edge that leaves the heavy member is skipped and reported."""
+    rng = np.random.default_rng(23)
+    sizes = [1500, 60001, 1024, 40000] + [1100] * 20
+    gs = mk.GraphSet(sizes, weighted=weighted)
+    off = gs.offsets.astype(np.int64)
+    mem = [_edges("random" if n != 40000 else "sparse", n, rng) for n in sizes]
+    s = np.concatenate([m[0] + off[i] for i, m in enumerate(mem)])
+    d = np.concatenate([m[1] + off[i] for i, m in enumerate(mem)])
+    w = to_dev(np.ones(len(s), np.uint32)) if weighted else None
+    gs.graph.InsertEdges(to_dev(s), to_dev(d), vals=w)
+    src = [int(m[0][0]) for m in mem]
+    bfs = mk.BFS(gs.graph, [int(off[i]) + src[i] for i in range(len(sizes))])
+    bfs.PrepareMembers([(int(off[i]), int(off[i + 1])) for i in range(len(sizes))])
+    for _ in range(2):
+        bfs.StaticMembers()
+        dist = bfs.Distances()
+        for i, (ms, md) in enumerate(mem):
+            O = OracleGraph(sizes[i])
+            O.insert(ms, md)
+            np.testing.assert_array_equal(dist[off[i]:off[i + 1]], O.bfs(src[i]))
+    assert gs.graph.sync() == 0
+    out = to_dev(np.array([off[1] + src[1]], np.uint32)), to_dev(np.array([off[0] + 1], np.uint32))
+    gs.graph.InsertEdges(*out, vals=to_dev(np.ones(1, np.uint32)) if weighted else None)
+    assert gs.graph.sync() == 0
+    before = dist[off[0]:off[1]]
+    bfs.StaticMembers()
+    np.testing.assert_array_equal(bfs.Distances()[off[0]:off[1]], before)
+    with pytest.raises(mk.MeerkatError, match="vertex id out of range"):
+        gs.graph.sync()
