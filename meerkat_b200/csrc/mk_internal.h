@@ -133,8 +133,6 @@ mk_status trav_member_bufs(mk_traversal *t, TravMemberBufs *out);
 // mk_bfs_static_members; wide_done (if given) is recorded behind the
 // device-wide part, before the member kernel.
 mk_status trav_static_members(mk_traversal *t, void *stream, float *ms_out, cudaEvent_t wide_done);
-// Whether some prepared member goes through the device-wide kernel.
-bool trav_members_wide(const mk_traversal *t);
 // Label array (one word per vertex) of a WCC handle.
 uint32_t *wcc_label_buf(mk_wcc *w);
 

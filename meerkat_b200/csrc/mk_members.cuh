@@ -177,7 +177,7 @@ __device__ __forceinline__ uint32_t ls_root(const uint16_t *p, uint32_t x) {
   return x;
 }
 
-__device__ __forceinline__ void ls_union(uint16_t *p, uint32_t a, uint32_t b, uint32_t *err) {
+static __device__ __noinline__ void ls_union(uint16_t *p, uint32_t a, uint32_t b, uint32_t *err) {
   for (uint32_t it = 0; it < kUfLimit; ++it) {
     const uint32_t ra = ls_find(p, a), rb = ls_find(p, b);
     if (ra == rb) return;
@@ -205,18 +205,19 @@ __device__ __forceinline__ void uf_member_link(const GraphView &g, const Lanes &
     for (uint32_t j = 0; j < kMemberHeads; ++j) own[j] = j < m ? __ldg(g.bowner + b + j) - lo : 0u;
     walk4_levels<kFused>(g, L, b, m, [&](uint32_t j, const uint4 x) {
       const uint32_t u = own[0] * (j == 0) + own[1] * (j == 1) + own[2] * (j == 2) + own[3] * (j == 3);
-      uint32_t k[4], w[4];
+      uint32_t k[4], w[4], need = 0;
       lane_keys<kW>(x, L.gl, k, w);
 #pragma unroll
       for (int t = 0; t < keys_per_lane<kW>(); ++t) {
         if (k[t] >= kTombKey) continue;
-        const uint32_t v = k[t] - lo;
-        if (v >= n || u >= n) {
+        k[t] -= lo;
+        if (k[t] >= n || u >= n)
           atomicOr(err, kErrInvalidId);
-          continue;
-        }
-        if (v != u) ls_union(sp, u, v, err);
+        else if (k[t] != u)
+          need |= 1u << t;
       }
+      for (; need; need &= need - 1)  // one call site: the walk copies this body eight times
+        ls_union(sp, u, need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3], err);
     });
   }
   __syncthreads();

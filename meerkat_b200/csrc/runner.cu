@@ -286,7 +286,7 @@ mk_status mk_set_runner_set_single(mk_set_runner *r, uint32_t on) {
 
 mk_status mk_set_runner_launches(mk_set_runner *r, uint32_t *h_launches) {
   if (!r || !h_launches) return fail(MK_ERR_INVALID, "mk_set_runner_launches: null argument");
-  *h_launches = r->single ? 1u : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u) + (trav_members_wide(r->bfs) ? 1u : 0u);
+  *h_launches = r->single ? 1u : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u);
   return MK_OK;
 }
 

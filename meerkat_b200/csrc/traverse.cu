@@ -409,7 +409,7 @@ __device__ __forceinline__ void expand_range(const TravArgs &a, const Lanes &L, 
 // hubs' lines stay there), what it lets through is tested again in L2, and
 // the one thread that sets the bit owns the vertex: a plain store of its
 // packed word, no atomic minimum and no stamp.
-template <bool kW>
+template <bool kW, bool kClosed>
 __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, const WarpQueue &Q,
                                              const uint4 (&q)[4], uint32_t nq, uint32_t u,
                                              uint32_t lo, uint32_t span, uint32_t lvl,
@@ -422,7 +422,7 @@ __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, 
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
       const bool live = (uint32_t)j < nq && k[j][i] < kTombKey;
-      const bool in = k[j][i] - lo < span;
+      const bool in = !kClosed || k[j][i] - lo < span;
       if (live && !in) atomicOr(a.g.err, kErrInvalidId);
       bits[j][i] = live && in ? __ldca(a.vis + (k[j][i] >> 5)) : ~0u;
     }
@@ -567,7 +567,9 @@ __device__ __forceinline__ void pull_reseed(const TravArgs &a, const Lanes &L, c
   }
 }
 
-template <bool kW, bool kUseW>
+// kClosed: the static BFS of graph-set members (TravArgs::closed); apart, since
+// its two words cost the plain BFS a fifth of its speed in spilled registers.
+template <bool kW, bool kUseW, bool kClosed>
 __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
   __shared__ uint32_t q_s[kTravWarps][kWarpQueue];
   __shared__ uint32_t qn_s[kTravWarps];
@@ -989,10 +991,10 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
           uint32_t u, b0, b1;
           item_range(a.g, now, a.chunk, u, b0, b1);
           if (!kUseW && a.vis) {
-            uint32_t lo, span;
-            closed_range(a, u, lo, span);
+            uint32_t lo = 0u, span = kTombKey;
+            if (kClosed) closed_range(a, u, lo, span);
             expand_range(a, L, b0, b1, [&](const uint4 (&q)[4], uint32_t nq) {
-              visit_slabs4<kW>(a, L, Q, q, nq, u, lo, span, lv, nxt, nsz);
+              visit_slabs4<kW, kClosed>(a, L, Q, q, nq, u, lo, span, lv, nxt, nsz);
             });
           } else {
             unsigned long long pu = 0;
@@ -1316,10 +1318,13 @@ static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, 
   a.treseed = t->rev ? t->treseed : nullptr;
   const void *fn;
   if (g->weighted)
-    fn = t->sssp ? (const void *)k_traverse<true, true> : (const void *)k_traverse<true, false>;
+    fn = t->sssp      ? (const void *)k_traverse<true, true, false>
+         : a.nclosed ? (const void *)k_traverse<true, false, true>
+                     : (const void *)k_traverse<true, false, false>;
   else
-    fn = (const void *)k_traverse<false, false>;
-  if (t->nblocks == 0) t->nblocks = persistent_blocks(fn, kTravBlock, 0, g->device);
+    fn = a.nclosed ? (const void *)k_traverse<false, false, true>
+                   : (const void *)k_traverse<false, false, false>;
+  if (t->nblocks == 0) t->nblocks = persistent_blocks(fn, kTravBlock, 0, g->device);  // the same for both forms: a block fills an SM
   void *args[] = {&a};
   MK_CUDA(cudaLaunchCooperativeKernel(fn, dim3(t->nblocks), dim3(kTravBlock), args, 0, s));
   return MK_OK;
@@ -1344,8 +1349,6 @@ static mk_status trav_launch(mk_traversal *t, uint32_t mode, const uint32_t *bs,
 }
 
 namespace mk {
-bool trav_members_wide(const mk_traversal *t) { return t && t->n_large != 0; }
-
 mk_status trav_member_bufs(mk_traversal *t, TravMemberBufs *out) {
   if (!t || !out) return fail(MK_ERR_INVALID, "trav_member_bufs: null argument");
   out->dist = t->dist;
