@@ -126,17 +126,19 @@ __device__ __forceinline__ void bfs_member(const GraphView &g, const Lanes &L, c
       const uint32_t ub0 = g.boff[gu], nb = g.boff[gu + 1] - ub0, cs = mem_chunk(nb);
       const uint32_t bb = ub0 + (item >> 16) * cs, be = min(bb + cs, ub0 + nb);
       auto relax = [&](const uint4 x) {
-        uint32_t k[4], w[4];
+        uint32_t k[4], w[4], need = 0;
         lane_keys<kW>(x, L.gl, k, w);
 #pragma unroll
         for (int t = 0; t < keys_per_lane<kW>(); ++t) {
           if (k[t] >= kTombKey) continue;
-          const uint32_t v = k[t] - lo;
-          if (v >= n) {
+          k[t] -= lo;
+          if (k[t] >= n)
             atomicOr(err, kErrInvalidId);
-            continue;
-          }
-          if ((vis[v >> 5] >> (v & 31)) & 1u) continue;
+          else if (!((vis[k[t] >> 5] >> (k[t] & 31)) & 1u))
+            need |= 1u << t;
+        }
+        for (; need; need &= need - 1) {  // one body: the walk copies this lambda eight times
+          const uint32_t v = need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3];
           if (cas_min16_first(par + v, u)) fl[atomicAdd(&s_nfound, 1u)] = v;
         }
       };

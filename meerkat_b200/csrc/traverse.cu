@@ -358,17 +358,30 @@ __device__ __forceinline__ void relax_slabs4(const TravArgs &a, const Lanes &L,
       cur[j][i] = live ? ld_dist(a.dist + v) : 0ull;
     }
   }
+  uint32_t need = 0;  // bit 4 j + i: key i of slab j looks improvable
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
-      const uint32_t v = k[j][i];
-      if (v == kEmptyKey) continue;
       const unsigned long long nd = (unsigned long long)du + (kUseW ? w[j][i] : 1u);
-      if (nd >= kInf || nd >= pack_hi(cur[j][i])) continue;
-      const unsigned long long old = atomicMin(a.dist + v, pack((uint32_t)nd, u));
-      if (pack_hi(old) > nd) push_improved(a, Q, nf, v, nd, stamp_next, gfr, gsz);
+      need |= (nd < kInf && nd < pack_hi(cur[j][i]) ? 1u : 0u) << (4 * j + i);  // no key: cur = 0
     }
+  // few keys get here: one body with the key picked by selects, instead of a
+  // copy per key
+  for (; need; need &= need - 1) {
+    const uint32_t at = __ffs(need) - 1;
+    uint32_t v = k[0][0], wt = w[0][0];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < KP; ++i)
+        if (at == 4u * j + i) {
+          v = k[j][i];
+          wt = w[j][i];
+        }
+    const uint32_t nd = du + (kUseW ? wt : 1u);
+    const unsigned long long old = atomicMin(a.dist + v, pack(nd, u));
+    if (pack_hi(old) > nd) push_improved(a, Q, nf, v, nd, stamp_next, gfr, gsz);
   }
 }
 
@@ -427,18 +440,28 @@ __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, 
       bits[j][i] = live && in ? __ldca(a.vis + (k[j][i] >> 5)) : ~0u;
     }
   }
+  uint32_t need = 0;  // bit 4 j + i: key i of slab j looks unvisited
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
+  for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int i = 0; i < KP; ++i) {
-      const uint32_t v = k[j][i], m = 1u << (v & 31);
-      if (bits[j][i] & m) continue;
-      uint32_t *word = a.vis + (v >> 5);
-      if (__ldcg(word) & m) continue;
-      if (atomicOr(word, m) & m) continue;
-      a.dist[v] = pack(lvl + 1, u);
-      push_vertex(a, Q, v, gfr, gsz);
-    }
+    for (int i = 0; i < KP; ++i)
+      need |= (((bits[j][i] >> (k[j][i] & 31)) & 1u) ^ 1u) << (4 * j + i);
+  // few keys get here: one body with the key picked by selects, instead of a
+  // copy per key (two walks of 16 keys outgrew the instruction cache)
+  for (; need; need &= need - 1) {
+    const uint32_t at = __ffs(need) - 1;
+    uint32_t v = k[0][0];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int i = 0; i < KP; ++i)
+        if (at == 4u * j + i) v = k[j][i];
+    const uint32_t m = 1u << (v & 31);
+    uint32_t *word = a.vis + (v >> 5);
+    if (__ldcg(word) & m) continue;
+    if (atomicOr(word, m) & m) continue;
+    a.dist[v] = pack(lvl + 1, u);
+    push_vertex(a, Q, v, gfr, gsz);
   }
 }
 
