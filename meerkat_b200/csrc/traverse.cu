@@ -870,16 +870,20 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
         uint32_t x, b0, b1;
         item_range(a.g, __ldcg(cur + i), a.chunk, x, b0, b1);
         walk_buckets(a.g, L, b0, b1, [&](const uint4 &q) {
-          uint32_t k[4], w[4];
+          uint32_t k[4], w[4], need = 0;
           lane_keys<kW>(q, L.gl, k, w);
+          // a child is told by its packed word alone: an invalidated vertex
+          // holds INFINF, and the one thread that sets its bit invalidates it
+          unsigned long long py[4];
 #pragma unroll
-          for (int j = 0; j < keys_per_lane<kW>(); ++j) {
-            uint32_t y = k[j];
-            if (y < kTombKey && y != x && !inval_test(a.inval, y)) {
-              unsigned long long py = ld_dist(a.dist + y);
-              if (py != kInfInf && !is_source(py, y) && pack_lo(py) == x && inval_set(a.inval, y))
-                invalidate(y, nxt, nsz);
-            }
+          for (int j = 0; j < keys_per_lane<kW>(); ++j)
+            py[j] = k[j] < kTombKey && k[j] != x ? ld_dist(a.dist + k[j]) : kInfInf;
+#pragma unroll
+          for (int j = 0; j < keys_per_lane<kW>(); ++j)
+            need |= (py[j] != kInfInf && pack_lo(py[j]) == x && !is_source(py[j], k[j]) ? 1u : 0u) << j;
+          for (; need; need &= need - 1) {
+            const uint32_t y = need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3];
+            if (inval_set(a.inval, y)) invalidate(y, nxt, nsz);
           }
         });
       }
@@ -942,16 +946,19 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
         walk4_set(a.g, L, bk, live, [&](uint32_t j, const uint4 q) {
           const uint32_t u = j == 0 ? u4[0] : j == 1 ? u4[1] : j == 2 ? u4[2] : u4[3];
           const uint32_t d = j == 0 ? d4[0] : j == 1 ? d4[1] : j == 2 ? d4[2] : d4[3];
-          uint32_t k[4], w[4], word[4];
+          uint32_t k[4], w[4], word[4], need = 0;
           lane_keys<kW>(q, L.gl, k, w);
 #pragma unroll
           for (int i = 0; i < keys_per_lane<kW>(); ++i)
             word[i] = k[i] < kTombKey ? __ldca(a.inval + (k[i] >> 5)) : 0u;
 #pragma unroll
-          for (int i = 0; i < keys_per_lane<kW>(); ++i) {
-            if (k[i] == u || !((word[i] >> (k[i] & 31)) & 1u)) continue;
-            relax(a, Q, all_near, k[i], (unsigned long long)d + (kUseW ? w[i] : 1u), u, round + 1,
-                  a.fr0, ctl + kSz0);
+          for (int i = 0; i < keys_per_lane<kW>(); ++i)
+            need |= (k[i] != u ? (word[i] >> (k[i] & 31)) & 1u : 0u) << i;
+          for (; need; need &= need - 1) {  // one body: the walk copies this lambda eight times
+            const uint32_t kt = need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3];
+            const uint32_t wt = need & 1u ? w[0] : need & 2u ? w[1] : need & 4u ? w[2] : w[3];
+            relax(a, Q, all_near, kt, (unsigned long long)d + (kUseW ? wt : 1u), u, round + 1, a.fr0,
+                  ctl + kSz0);
           }
         });
       }

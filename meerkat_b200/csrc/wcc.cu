@@ -221,10 +221,14 @@ __global__ void k_uf_sample(GraphView g, uint32_t *p, const uint32_t *sel_bits, 
           k1[j] = k;
       }
     }
-#pragma unroll
-    for (uint32_t j = 0; j < 4; ++j) {
-      if (k0[j] < kTombKey) uf_union(p, uu[j], k0[j], err, fe);
-      if (k1[j] < kTombKey) uf_union(p, uu[j], k1[j], err, fe);
+#pragma unroll 1
+    for (uint32_t i = 0; i < 8; ++i) {  // one copy of the union
+      const uint32_t j = i >> 1;
+      const uint32_t u = j == 0 ? uu[0] : j == 1 ? uu[1] : j == 2 ? uu[2] : uu[3];
+      const uint32_t a0 = j == 0 ? k0[0] : j == 1 ? k0[1] : j == 2 ? k0[2] : k0[3];
+      const uint32_t a1 = j == 0 ? k1[0] : j == 1 ? k1[1] : j == 2 ? k1[2] : k1[3];
+      const uint32_t v = (i & 1u) ? a1 : a0;
+      if (v < kTombKey) uf_union(p, u, v, err, fe);
     }
   }
 }
@@ -797,18 +801,21 @@ __global__ void k_uf_scan_items(GraphView g, uint32_t *p, const uint32_t *items,
         uint32_t pj = px[0] * (j == 0) + px[1] * (j == 1) + px[2] * (j == 2) + px[3] * (j == 3);
         uint32_t k[4], w[4];
         lane_keys<kW>(q, L.gl, k, w);
-        uint32_t py[4];
+        uint32_t py[4] = {0u, 0u, 0u, 0u};
         bool ok[4];
 #pragma unroll
         for (int t = 0; t < keys_per_lane<kW>(); ++t) {
           ok[t] = k[t] < kTombKey && k[t] != x && k[t] < g.V;
           py[t] = ok[t] ? __ldcg(p + k[t]) : 0u;
         }
+        uint32_t need = 0;
 #pragma unroll
-        for (int t = 0; t < keys_per_lane<kW>(); ++t) {
-          if (!ok[t] || py[t] == pj) continue;
+        for (int t = 0; t < keys_per_lane<kW>(); ++t) need |= (ok[t] && py[t] != pj ? 1u : 0u) << t;
+        for (; need; need &= need - 1) {
+          const uint32_t kt = need & 1u ? k[0] : need & 2u ? k[1] : need & 4u ? k[2] : k[3];
+          const uint32_t pt = need & 1u ? py[0] : need & 2u ? py[1] : need & 4u ? py[2] : py[3];
           // kIn: the slab edge k -> x of the graph
-          pj = kIn ? uf_union_root(p, k[t], x, err, fe) : uf_union_root(p, x, k[t], err, fe);
+          if (pt != pj) pj = kIn ? uf_union_root(p, kt, x, err, fe) : uf_union_root(p, x, kt, err, fe);
         }
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i)
