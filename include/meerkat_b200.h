@@ -348,7 +348,9 @@ mk_status mk_pagerank_stats(mk_pagerank *p, uint32_t *h_iters,
 mk_status mk_pagerank_destroy(mk_pagerank *p);
 
 /* PageRank of one vertex range of an OUT-edge graph (a graph-set member),
- * push form, FP64 accumulation: no reverse graph needed.  Same formula,
+ * FP64 accumulation: no reverse graph needed.  A run turns the member's live
+ * edges around in scratch (8 bytes per edge, kept by the handle; pushed
+ * straight from the slabs where that does not fit).  Same formula,
  * start and stopping rule as above with N = v_end - v_begin; out-degrees are
  * the graph's live degrees.  The range must be closed under out-edges.
  * No counterpart in the reference (whose PageRank needs the reverse graph). */

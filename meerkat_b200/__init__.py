@@ -464,8 +464,8 @@ class PageRank(_Timed):
 
 
 class PageRankRange(_Timed):
-    """PageRank of one vertex range (a GraphSet member) of an out-edge graph,
-    push form: no reverse graph needed (mk_pagerank_range_*)."""
+    """PageRank of one vertex range (a GraphSet member) of an out-edge graph:
+    no reverse graph needed (mk_pagerank_range_*)."""
 
     def __init__(self, G: DynamicGraph, max_vertices: int):
         self.G = G

@@ -115,7 +115,7 @@ def tune_frontier_chunk(G, traversal, chunks: Sequence[int] = CHUNKS, repeats: i
     return {"best": best["frontier_chunk"], "trials": trials}
 
 
-# static SSSP near-far steps (0 = plain level-synchronous)
+# static SSSP near-far steps (0 = automatic: the threshold doubles)
 SSSP_DELTAS: Tuple[int, ...] = (0, 128, 512, 2048, 8192)
 
 

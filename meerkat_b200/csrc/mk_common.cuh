@@ -119,7 +119,9 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t *p) {
 // barrier is over once every block has arrived as often as this one, so an
 // arrival is one fire-and-forget add and nothing is reset between barriers
 // (the count wraps: compared as a signed difference).  One arrival and one
-// poller per block: launch few large blocks.  The wait is bounded by
+// poller per block: launch few large blocks.  The poll is relaxed, with one
+// fence behind it: an acquiring poll drops the SM's L1 lines on every spin,
+// under the other blocks that are still working there.  The wait is bounded by
 // `limit_ns`; on expiry the kernel's error word gets kErrTimeout and sync
 // returns false so every block can leave.
 struct GridBarrier {
@@ -142,7 +144,7 @@ struct GridBarrier {
       // is honoured; another block's timeout is noticed within 16 spins
       const unsigned long long t0 = global_ns();
       uint32_t spins = 0;
-      while ((int32_t)(ld_acquire_u32(bar) - target) < 0) {
+      while ((int32_t)(ld_relaxed_u32(bar) - target) < 0) {
         if (global_ns() - t0 > limit_ns) {
           atomicOr(err, kErrTimeout);
           ok = 0;
@@ -153,6 +155,8 @@ struct GridBarrier {
           break;
         }
       }
+      // the acquire: with the arrivals' fences before their adds, everything
+      // written before the barrier is visible behind it
       __threadfence();
       ok_s = ok;
     }

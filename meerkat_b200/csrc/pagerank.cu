@@ -185,20 +185,19 @@ constexpr uint32_t kPrFlat = 256;   // in-degree up to which the flat pass sums 
 constexpr uint32_t kPrChunk = 256;  // in-edges per work item of a hub (in-degree > kPrFlat)
 constexpr int kPrSteps = 4;         // 32-edge steps of the flat pass whose loads are in flight together
 
-// Segmented inclusive sum across the warp: lanes with equal keys form
-// contiguous runs, and each lane ends with the sum of its run up to itself
-// (a fixed tree order).
-__device__ __forceinline__ float seg_scan(float v, uint32_t key, uint32_t lane) {
+// Segmented inclusive sum across the warp: each lane ends with the sum of its
+// run up to itself (a fixed tree order); `in` is the lane's position in its
+// run, so no keys are compared or shuffled.
+__device__ __forceinline__ float seg_scan(float v, uint32_t in) {
 #pragma unroll
   for (int s = 1; s < 32; s <<= 1) {
     const float y = __shfl_up_sync(0xFFFFFFFFu, v, s);
-    const uint32_t ky = __shfl_up_sync(0xFFFFFFFFu, key, s);
-    if (lane >= (uint32_t)s && ky == key) v += y;
+    if (in >= (uint32_t)s) v += y;
   }
   return v;
 }
 
-__global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
+__global__ void __launch_bounds__(kPrBlock, 3) k_pagerank(PrArgs a) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t nthreads = gridDim.x * blockDim.x;
   const uint32_t lane = threadIdx.x & 31u;
@@ -292,27 +291,33 @@ __global__ void __launch_bounds__(kPrBlock) k_pagerank(PrArgs a) {
       const unsigned long long basej = j0 - off;  // edge x of the run of lane l is col[basej(l) + x]
       Kahan acc;
       for (uint32_t t0 = 0; t0 < T; t0 += 32u * kPrSteps) {
-        uint32_t own[kPrSteps], kc[kPrSteps];
+        uint32_t in[kPrSteps], kc[kPrSteps];  // position in the run, column
         float val[kPrSteps];
 #pragma unroll
         for (int q = 0; q < kPrSteps; ++q) {
           const uint32_t x = t0 + 32u * q + lane;
-          uint32_t lo = 0;  // last lane whose run starts at or before x
+          uint32_t lo = 0, from = 0;  // last lane whose run starts at or before x, and where it does
 #pragma unroll
           for (int st = 16; st > 0; st >>= 1) {
             const uint32_t cand = lo + (uint32_t)st;
-            if (__shfl_sync(0xFFFFFFFFu, off, cand) <= x) lo = cand;
+            const uint32_t o = __shfl_sync(0xFFFFFFFFu, off, cand);
+            if (o <= x) {
+              lo = cand;
+              from = o;
+            }
           }
           const unsigned long long bj = __shfl_sync(0xFFFFFFFFu, basej, lo);
-          own[q] = x < T ? lo : 32u;
+          in[q] = min(lane, x - from);  // of the part of the run in this step
           kc[q] = x < T ? __ldcs(a.col + (bj + x)) : 0u;
         }
 #pragma unroll
-        for (int q = 0; q < kPrSteps; ++q) val[q] = own[q] < 32u ? __ldca(c + kc[q]) : 0.0f;
+        for (int q = 0; q < kPrSteps; ++q)
+          val[q] = t0 + 32u * q + lane < T ? __ldca(c + kc[q]) : 0.0f;
 #pragma unroll
         for (int q = 0; q < kPrSteps; ++q) {
-          const float sv = seg_scan(val[q], own[q], lane);
           const uint32_t sb = t0 + 32u * q;
+          if (sb >= T) break;  // uniform: no run reaches here
+          const float sv = seg_scan(val[q], in[q]);
           const bool hit = dl && off < sb + 32u && off + dl > sb;
           const uint32_t last = hit ? min(off + dl, sb + 32u) - 1u - sb : 0u;
           const float tot = __shfl_sync(0xFFFFFFFFu, sv, last);

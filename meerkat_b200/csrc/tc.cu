@@ -248,12 +248,14 @@ __global__ void k_tc_own(uint32_t V, const unsigned long long *__restrict__ orow
 // Per-owner work is heavy-tailed, so owners are split into chunks and handed
 // out dynamically.  Owners whose list is longer than kTcSmallMax go to the
 // big list instead.
-__global__ void k_tc_item_count(uint32_t V, const uint32_t *__restrict__ odeg,
+__global__ void k_tc_item_count(uint32_t V, const unsigned long long *__restrict__ orow,
                                 const unsigned long long *__restrict__ prow,
+                                uint32_t *__restrict__ odeg,
                                 uint32_t *__restrict__ icnt, uint32_t *big_list, uint32_t *big_n,
                                 uint32_t *big_max) {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x) {
-    const uint32_t du = odeg[u], np = (uint32_t)(prow[u + 1] - prow[u]);
+    const uint32_t du = (uint32_t)(orow[u + 1] - orow[u]), np = (uint32_t)(prow[u + 1] - prow[u]);
+    odeg[u] = du;
     uint32_t c = 0;
     if (du && np) {
       if (du > kTcSmallMax) {
@@ -648,6 +650,12 @@ struct mk_tc {
   Timer timer;
 };
 
+// Edges from which the static counts sort them by owner: the sort is seven
+// more launches, which pay from about half a million edges (100,000 oriented
+// ones: 162 -> 205 us with it; a million: 423 -> 415 us; 7.5 million: 5.5 ->
+// 2.9 ms).
+constexpr unsigned long long kOwnEdges = 1u << 19;
+
 // Arrays of the counting pass that hold the list lengths (V words), the
 // edges by owner (a word per oriented edge) and their rows (V + 1).
 struct TcOwners {
@@ -698,10 +706,10 @@ static mk_status tc_static(mk_tc *t, cudaStream_t s) {
   MK_CHECK(t->odeg.reserve(V, &acc));
   TcOwners own{t->odeg.ptr, nullptr, nullptr, nullptr};
   // without room for the edges by owner, every edge stays with its lower end
-  if (t->pcol.reserve(std::max<unsigned long long>(total, 1), &acc) == MK_OK &&
+  if (total >= kOwnEdges && t->pcol.reserve(std::max<unsigned long long>(total, 1), &acc) == MK_OK &&
       t->prow.reserve((size_t)V + 1, &acc) == MK_OK && t->pcnt.reserve(V, &acc) == MK_OK)
     own = {t->odeg.ptr, t->pcnt.ptr, t->pcol.ptr, t->prow.ptr};
-  else
+  else if (total >= kOwnEdges)
     (void)cudaGetLastError();
   return tc_count_oriented(t, V, g->device, own, s);
 }
@@ -714,18 +722,16 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, TcOwners ow
   size_t acc = 0;
   const unsigned long long *prow = t->orow.ptr;
   const uint32_t *pcol = t->ocol.ptr;
-  {
+  if (own.pcol) {
     const int vb = (int)std::min<uint64_t>((uint64_t)V / 256 + 1, (uint64_t)device_sm_count(device) * 8);
+    const int gb = groups_grid(V, device);
     k_tc_odeg<<<vb, 256, 0, s>>>(V, t->orow.ptr, own.odeg);
-    if (own.pcol) {
-      const int gb = groups_grid(V, device);
-      MK_CUDA(cudaMemsetAsync(own.pcnt, 0, (size_t)V * 4, s));
-      k_tc_own<false><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, nullptr, nullptr);
-      MK_CHECK(scan_u32_to_u64(own.pcnt, own.prow, V, t->tmp, s));
-      k_tc_own<true><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, own.prow, own.pcol);
-      prow = own.prow;
-      pcol = own.pcol;
-    }
+    MK_CUDA(cudaMemsetAsync(own.pcnt, 0, (size_t)V * 4, s));
+    k_tc_own<false><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, nullptr, nullptr);
+    MK_CHECK(scan_u32_to_u64(own.pcnt, own.prow, V, t->tmp, s));
+    k_tc_own<true><<<gb, 256, 0, s>>>(V, t->orow.ptr, t->ocol.ptr, own.odeg, own.pcnt, own.prow, own.pcol);
+    prow = own.prow;
+    pcol = own.pcol;
   }
   MK_CHECK(t->big_list.reserve(V, &acc));
   MK_CUDA(cudaMemsetAsync(t->dcount, 0, 8, s));
@@ -734,7 +740,7 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, TcOwners ow
   // work items (the orientation scratch is free again: ocnt >= V words,
   // bpos >= V + 1)
   const int vb = (int)std::min<uint64_t>((uint64_t)V / 256 + 1, (uint64_t)device_sm_count(device) * 8);
-  k_tc_item_count<<<vb, 256, 0, s>>>(V, own.odeg, prow, t->ocnt.ptr, t->big_list.ptr, t->small,
+  k_tc_item_count<<<vb, 256, 0, s>>>(V, t->orow.ptr, prow, own.odeg, t->ocnt.ptr, t->big_list.ptr, t->small,
                                      t->small + 2);
   MK_CHECK(scan_u32_to_u64(t->ocnt.ptr, t->bpos.ptr, V, t->tmp, s));
   unsigned long long nitems = 0;
@@ -937,7 +943,8 @@ mk_status mk_tc_range_run(mk_tc_range *t, uint32_t v_begin, uint32_t v_end, void
   MK_CUDA(cudaGetLastError());
   // the member's CSR rows, row ids and degree counts are done with: they hold
   // the edges by owner
-  const TcOwners own{t->recip.ptr, t->indeg.ptr, t->rowid.ptr, t->rp.ptr};
+  TcOwners own{t->recip.ptr, t->indeg.ptr, t->rowid.ptr, t->rp.ptr};
+  if (E < kOwnEdges) own.pcol = nullptr;
   MK_CHECK(tc_count_oriented(c, n, g->device, own, s));
   return c->timer.stop(ms_out);
 }

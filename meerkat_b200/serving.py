@@ -15,7 +15,7 @@ scheduling round takes the oldest pending request of every free graph:
 
 These fast segments are issued on one CUDA stream without waiting for the
 device; a CUDA event after each segment marks its requests complete.
-PageRank (push form on the member's out-edges, mk_pagerank_range_*) and
+PageRank (from the member's out-edges, mk_pagerank_range_*) and
 triangle counting (straight from the member's out-edges, mk_tc_range_*) are
 heavy: a worker thread runs them one at a time on a second stream, so they
 overlap the fast rounds instead of holding them up.
@@ -239,6 +239,10 @@ class GraphServer:
         # (a later growth would synchronise the device mid-run)
         edges = [int(self.G.count_edges(lo, hi)) for lo, hi in ranges]
         big = int(np.argmax(edges))
+        # the range PageRank's turned edges and per-vertex words (its buffers
+        # grow in powers of two); it pushes from the slabs where they do not fit
+        pow2 = lambda n: 1 << max(10, (int(n) - 1).bit_length())  # noqa: E731
+        self.resident += 8 * pow2(max(edges)) + 20 * pow2(sizes.max())
         warm = Request(rid=-1, graph=big, kind=TC_Q, arrival=0.0)
         self.run_heavy(warm, self.heavy)
         if warm.status != "ok":
