@@ -186,17 +186,30 @@ constexpr uint32_t kPrChunk = 256;  // in-edges per work item of a hub (in-degre
 constexpr int kPrSteps = 4;         // 32-edge steps of the flat pass whose loads are in flight together
 
 // Segmented inclusive sum across the warp: each lane ends with the sum of its
-// run up to itself (a fixed tree order); `in` is the lane's position in its
-// run, so no keys are compared or shuffled.
-__device__ __forceinline__ float seg_scan(float v, uint32_t in) {
+// run up to itself (a fixed tree order, the same in both forms).  kPos: tag
+// is the lane's position in its run, so no keys are shuffled, which frees the
+// pipe the gathers share (32 M edges: 3.86 -> 3.52 ms); else tag is the run's
+// key, whose compares wait on nothing before them: a solve of few edges is
+// bound by each warp's own latency (2.4 M edges: 0.86 against 0.89 ms,
+// 240,000: 0.55 against 0.60).
+template <bool kPos>
+__device__ __forceinline__ float seg_scan(float v, uint32_t tag, uint32_t lane) {
 #pragma unroll
   for (int s = 1; s < 32; s <<= 1) {
     const float y = __shfl_up_sync(0xFFFFFFFFu, v, s);
-    if (in >= (uint32_t)s) v += y;
+    if (kPos) {
+      if (tag >= (uint32_t)s) v += y;
+    } else {
+      const uint32_t ky = __shfl_up_sync(0xFFFFFFFFu, tag, s);
+      if (lane >= (uint32_t)s && ky == tag) v += y;
+    }
   }
   return v;
 }
 
+constexpr unsigned long long kPrPosEdges = 8ull << 20;  // edges from which runs are told by position
+
+template <bool kPos>
 __global__ void __launch_bounds__(kPrBlock, 3) k_pagerank(PrArgs a) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t nthreads = gridDim.x * blockDim.x;
@@ -291,7 +304,7 @@ __global__ void __launch_bounds__(kPrBlock, 3) k_pagerank(PrArgs a) {
       const unsigned long long basej = j0 - off;  // edge x of the run of lane l is col[basej(l) + x]
       Kahan acc;
       for (uint32_t t0 = 0; t0 < T; t0 += 32u * kPrSteps) {
-        uint32_t in[kPrSteps], kc[kPrSteps];  // position in the run, column
+        uint32_t tag[kPrSteps], kc[kPrSteps];  // seg_scan's tag, column
         float val[kPrSteps];
 #pragma unroll
         for (int q = 0; q < kPrSteps; ++q) {
@@ -307,7 +320,7 @@ __global__ void __launch_bounds__(kPrBlock, 3) k_pagerank(PrArgs a) {
             }
           }
           const unsigned long long bj = __shfl_sync(0xFFFFFFFFu, basej, lo);
-          in[q] = min(lane, x - from);  // of the part of the run in this step
+          tag[q] = kPos ? min(lane, x - from) : x < T ? lo : 32u;
           kc[q] = x < T ? __ldcs(a.col + (bj + x)) : 0u;
         }
 #pragma unroll
@@ -316,8 +329,7 @@ __global__ void __launch_bounds__(kPrBlock, 3) k_pagerank(PrArgs a) {
 #pragma unroll
         for (int q = 0; q < kPrSteps; ++q) {
           const uint32_t sb = t0 + 32u * q;
-          if (sb >= T) break;  // uniform: no run reaches here
-          const float sv = seg_scan(val[q], in[q]);
+          const float sv = seg_scan<kPos>(val[q], tag[q], lane);
           const bool hit = dl && off < sb + 32u && off + dl > sb;
           const uint32_t last = hit ? min(off + dl, sb + 32u) - 1u - sb : 0u;
           const float tot = __shfl_sync(0xFFFFFFFFu, sv, last);
@@ -471,6 +483,7 @@ struct mk_pagerank {
   DevBuf<uint32_t> col, cnt, mflag, item_v, multi, gcnt;
   DevBuf<float> ipart;
   uint32_t *ctl = nullptr;
+  uint64_t edges = 0;  // of the CSR of this solve
   uint32_t cur = 0;  // host mirror of the buffer with the latest ranks
   int nblocks = 0;
   Timer timer;
@@ -494,6 +507,7 @@ static mk_status pr_prepare(mk_pagerank *p, cudaStream_t s) {
   const uint32_t V = g->V;
   uint64_t E = 0;
   MK_CHECK(export_csr_grow(g, p->rp, p->col, s, &E, nullptr));
+  p->edges = E;
   MK_CHECK(p->cnt.reserve(V));
   MK_CHECK(p->mflag.reserve(V));
   MK_CHECK(p->ioff.reserve((size_t)V + 1));
@@ -525,7 +539,9 @@ static mk_status pr_prepare(mk_pagerank *p, cudaStream_t s) {
 // solve pays for it inside its timed window.
 static mk_status pr_setup_launch(mk_pagerank *p) {
   if (p->nblocks) return MK_OK;
-  const int nb = persistent_blocks((const void *)k_pagerank, kPrBlock, 0, p->g->device);
+  // the same grid for both forms
+  const int nb = std::min(persistent_blocks((const void *)k_pagerank<true>, kPrBlock, 0, p->g->device),
+                          persistent_blocks((const void *)k_pagerank<false>, kPrBlock, 0, p->g->device));
   cudaError_t e = cudaMalloc(&p->part, (size_t)nb * 8 * sizeof(float));
   if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(pagerank partials)");
   p->nblocks = nb;
@@ -535,7 +551,7 @@ static mk_status pr_setup_launch(mk_pagerank *p) {
 static mk_status pr_solve(mk_pagerank *p, cudaStream_t s) {
   mk_graph *g = p->g;
   MK_CHECK(pr_prepare(p, s));
-  const void *fn = (const void *)k_pagerank;
+  const void *fn = p->edges >= kPrPosEdges ? (const void *)k_pagerank<true> : (const void *)k_pagerank<false>;
   MK_CHECK(pr_setup_launch(p));
   MK_CUDA(cudaMemsetAsync(p->ctl, 0, kPCtlWords * 4, s));
   PrArgs a;

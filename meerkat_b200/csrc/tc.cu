@@ -181,7 +181,7 @@ __device__ __noinline__ uint32_t bucket_probe_on(const uint4 *set, uint32_t nb, 
   return 0u;
 }
 
-constexpr uint32_t kTcChunk = 64;  // partners per work item
+constexpr uint32_t kTcChunk = 32;  // partners per work item (one per lane)
 constexpr int kTcSteps = 4;        // 32-entry probe steps with their loads in flight together
 
 // Length of every oriented list.
@@ -244,7 +244,7 @@ __global__ void k_tc_own(uint32_t V, const unsigned long long *__restrict__ orow
   }
 }
 
-// Work items: (h, chunk c) covers partners [64 c, 64 c + 64) of owner h.
+// Work items: (h, chunk c) covers partners [32 c, 32 c + 32) of owner h.
 // Per-owner work is heavy-tailed, so owners are split into chunks and handed
 // out dynamically.  Owners whose list is longer than kTcSmallMax go to the
 // big list instead.
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kTcWarps * 32)
     }
     const unsigned long long p0 = prow[u] + (unsigned long long)chunk * kTcChunk;
     const unsigned long long pe = prow[u + 1];
-    uint32_t c = 0;  // this item's triangles found by the lane (at most 64 lists of 2^32 / 32 entries)
+    uint32_t c = 0;  // this item's triangles found by the lane (at most 32 lists of 2^32 / 32 entries)
     for (unsigned long long pb = p0; pb < p0 + kTcChunk && pb < pe; pb += 32) {
       const uint32_t m = pe - pb < 32 ? (uint32_t)(pe - pb) : 32u;
       // one partner's list per lane, handed round below
