@@ -195,7 +195,8 @@ typedef struct mk_tuning {
                                     distances >= threshold wait on a far list
                                     until the near frontier drains, then the
                                     threshold moves on by this much; 0 =
-                                    automatic (it doubles)                     */
+                                    automatic (it doubles; below a million
+                                    buckets no split)                          */
   uint32_t recompute_permille;   /* decremental BFS/SSSP: once this share of
                                     the vertices (per mille) is invalidated,
                                     recompute from the sources instead of
@@ -562,7 +563,9 @@ mk_status mk_gen_set_batches(const uint32_t *d_vertex_offsets, uint32_t num_grap
  * components) or MK_QUERY_NONE.  create uploads the query tables (blocking).
  * step applies one update batch covering any members (deletes, then inserts;
  * global vertex ids, device arrays; d_ins_w may be NULL) and then answers
- * every member's query: four launches, all asynchronous on `stream` and
+ * every member's query: four launches (one more when a member outweighs the
+ * others), all asynchronous, ordered on `stream` (the components run beside
+ * the BFS on a stream of the runner's own that joins it) and
  * allocation-free once mk_graph_reserve_batch has sized the batch scratch,
  * so a step can be captured into a CUDA graph.  A member's answers equal
  * those of a DynamicGraph holding the member alone (an edge leaving its
