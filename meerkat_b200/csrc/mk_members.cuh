@@ -179,7 +179,7 @@ __device__ __forceinline__ uint32_t ls_root(const uint16_t *p, uint32_t x) {
   return x;
 }
 
-static __device__ __noinline__ void ls_union(uint16_t *p, uint32_t a, uint32_t b, uint32_t *err) {
+__device__ __forceinline__ void ls_union(uint16_t *p, uint32_t a, uint32_t b, uint32_t *err) {
   for (uint32_t it = 0; it < kUfLimit; ++it) {
     const uint32_t ra = ls_find(p, a), rb = ls_find(p, b);
     if (ra == rb) return;
