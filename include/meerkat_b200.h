@@ -353,7 +353,9 @@ mk_status mk_pagerank_destroy(mk_pagerank *p);
  * edges around in scratch (8 bytes per edge, kept by the handle; pushed
  * straight from the slabs where that does not fit).  Same formula,
  * start and stopping rule as above with N = v_end - v_begin; out-degrees are
- * the graph's live degrees.  The range must be closed under out-edges.
+ * the graph's live degrees.  The range must be closed under out-edges, and
+ * its edges must not change during the run (order updates before it or after
+ * it); a run that they change under ends with approximate ranks.
  * No counterpart in the reference (whose PageRank needs the reverse graph). */
 typedef struct mk_pagerank_range mk_pagerank_range;
 mk_status mk_pagerank_range_create(mk_graph *g, uint32_t max_vertices,

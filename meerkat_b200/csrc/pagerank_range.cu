@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "mk_internal.h"
+#include "mk_rows.h"
 #include "mk_slab.cuh"
 
 namespace mk {
@@ -110,7 +111,8 @@ constexpr uint32_t kPrrSteps = 4;    // 32-pair steps whose loads are in flight 
 // Live edges per target of the range (fill false), or the pairs written at
 // their targets' positions, the counts used up as cursors (fill true).  A key
 // outside the range (a range that is not closed under edges) is skipped and
-// reported as MK_DEVERR_INVALID_ID.
+// reported as MK_DEVERR_INVALID_ID.  An edge that was not counted (the member
+// changed under the call) is left out (row_place).
 template <bool kW, bool kFill>
 __global__ void k_prr_turn(GraphView g, uint32_t lo, uint32_t n, uint32_t b0, uint32_t nb,
                            uint32_t *__restrict__ cnt, const unsigned long long *__restrict__ rp,
@@ -139,9 +141,8 @@ __global__ void k_prr_turn(GraphView g, uint32_t lo, uint32_t n, uint32_t b0, ui
         } else if (!kFill) {
           atomicAdd(cnt + v, 1u);
         } else {
-          const uint32_t left = atomicSub(cnt + v, 1u);
-          at[t] = left - 1u;
-          if (left == 0) k[t] = kEmptyKey;  // not counted: the graph changed under the call
+          at[t] = row_place(atomicSub(cnt + v, 1u), rp[v + 1] - rp[v]);
+          if (at[t] == kNoPlace) k[t] = kEmptyKey;
         }
       }
       if (!kFill) return;
@@ -152,10 +153,13 @@ __global__ void k_prr_turn(GraphView g, uint32_t lo, uint32_t n, uint32_t b0, ui
   }
 }
 
-// PR = x, the first contributions, empty sums, the first dangling mass.
+// PR = x, the first contributions, empty sums, the first dangling mass; and
+// the places that the fill left open (edges that went between the count and
+// the fill) get no target, so the gather never follows an old word.
 __global__ void k_prr_start(double *__restrict__ pr, double *__restrict__ c, double *__restrict__ sum,
                             const uint32_t *__restrict__ deg, uint32_t n, double x, double d,
-                            double *dang) {
+                            double *dang, const uint32_t *__restrict__ cnt,
+                            const unsigned long long *__restrict__ rp, uint2 *__restrict__ pairs) {
   double lost = 0.0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t dg = deg[i];
@@ -163,6 +167,11 @@ __global__ void k_prr_start(double *__restrict__ pr, double *__restrict__ c, dou
     sum[i] = 0.0;
     c[i] = dg ? d * x / (double)dg : 0.0;
     if (!dg) lost += x;
+    const uint32_t left = cnt[i];
+    if (left) {
+      const unsigned long long r0 = rp[i], gap = row_gap(left, rp[i + 1] - r0);
+      for (unsigned long long j = 0; j < gap; ++j) pairs[r0 + j] = make_uint2(0u, kEmptyKey);
+    }
   }
   block_add(lost, dang);
 }
@@ -197,10 +206,9 @@ __global__ void __launch_bounds__(256)
       for (uint32_t r = 0; r < kPrrSteps; ++r) val[r] = p[r].y != kEmptyKey ? __ldg(c + p[r].x) : 0.0;
 #pragma unroll
       for (uint32_t r = 0; r < kPrrSteps; ++r) {
-        const uint32_t key = p[r].y;
+        if (s0 + 32u * r >= e1) break;
+        const uint32_t key = p[r].y;  // kEmptyKey: no edge here, val 0
         double v = val[r];
-        const uint32_t first = __shfl_sync(0xFFFFFFFFu, key, 0);
-        if (first == kEmptyKey) break;  // past the end (uniform)
         if (lane == 0) {
           if (key == ckey)
             v += cval;
@@ -215,7 +223,7 @@ __global__ void __launch_bounds__(256)
         }
         const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, key, 1);
         if (lane < 31 && key != next && key != kEmptyKey) atomicAdd(sum + key, v);
-        ckey = __shfl_sync(0xFFFFFFFFu, key, 31);  // empty when the chunk ended in this step
+        ckey = __shfl_sync(0xFFFFFFFFu, key, 31);  // kEmptyKey when the chunk ended in this step
         cval = __shfl_sync(0xFFFFFFFFu, v, 31);
       }
     }
@@ -350,7 +358,8 @@ static mk_status prr_gather_solve(mk_pagerank_range *p, uint32_t lo, uint32_t n,
       1, std::min<uint64_t>((chunks + 7) / 8, (uint64_t)device_sm_count(g->device) * 8));
   double *dang = p->acc, *delta = p->acc + kPrrBatch + 1;
   MK_CUDA(cudaMemsetAsync(p->acc, 0, (2 * kPrrBatch + 1) * 8, s));
-  k_prr_start<<<fb, 256, 0, s>>>(p->a, p->c.ptr, p->b, deg, n, 1.0 / n, d, dang);
+  k_prr_start<<<fb, 256, 0, s>>>(p->a, p->c.ptr, p->b, deg, n, 1.0 / n, d, dang, p->cnt.ptr, p->rp.ptr,
+                                 p->pairs.ptr);
   MK_CUDA(cudaGetLastError());
   uint32_t it = 0;
   double h[kPrrBatch];
