@@ -350,8 +350,9 @@ mk_status mk_pagerank_destroy(mk_pagerank *p);
 
 /* PageRank of one vertex range of an OUT-edge graph (a graph-set member),
  * FP64 accumulation: no reverse graph needed.  A run turns the member's live
- * edges around in scratch (8 bytes per edge, kept by the handle; pushed
- * straight from the slabs where that does not fit).  Same formula,
+ * edges around in scratch (8 bytes per edge, kept by the handle; runs of at
+ * most three iterations, and those that it does not fit for, push straight
+ * from the slabs).  Same formula,
  * start and stopping rule as above with N = v_end - v_begin; out-degrees are
  * the graph's live degrees.  The range must be closed under out-edges, and
  * its edges must not change during the run (order updates before it or after

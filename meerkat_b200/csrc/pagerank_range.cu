@@ -21,10 +21,10 @@
 //           mass of the next iteration.
 // What bounds it: the pairs stream from L2 (8 bytes an edge) and the gathers
 // of the contributions (8 bytes each, mostly L2).  Pushing straight from the
-// slabs (k_prr_push, kept for when the pairs do not fit in memory) walked
-// every 128-byte line and issued an atomic per edge in every iteration: 107 us
-// an iteration at 262,144 vertices and 4.1 M weighted edges, five launches and
-// a host round trip each.
+// slabs (k_prr_push) walks every 128-byte line and issues an atomic per edge
+// in every iteration: about 130 us an iteration at 262,144 vertices and 4.1 M
+// weighted edges, five launches and a host round trip each.  It stays for runs
+// of few iterations and for when the pairs do not fit in memory.
 // The device decides when to stop: iterations are issued kPrrBatch at a time,
 // a launch behind the converged one returns at once, and the host reads the
 // deltas once per batch.  FP64 accumulation keeps the result within the same
@@ -82,8 +82,10 @@ __global__ void k_prr_base(double *__restrict__ nx, uint32_t n, const double *ac
     nx[i] = base;
 }
 
+// One iteration straight from the slabs: an atomic per live edge.  A key
+// outside the range is skipped and reported, as k_prr_turn does.
 template <bool kW>
-__global__ void k_prr_push(GraphView g, uint32_t lo, uint32_t b0, uint32_t nb,
+__global__ void k_prr_push(GraphView g, uint32_t lo, uint32_t n, uint32_t b0, uint32_t nb,
                            const double *__restrict__ pr, double *nx, double d) {
   const Lanes L = lanes();
   const uint32_t group = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
@@ -98,12 +100,23 @@ __global__ void k_prr_push(GraphView g, uint32_t lo, uint32_t b0, uint32_t nb,
       uint32_t k[4], w[4];
       lane_keys<kW>(q, L.gl, k, w);
 #pragma unroll
-      for (int j = 0; j < keys_per_lane<kW>(); ++j)
-        if (k[j] < kTombKey) atomicAdd(nx + (k[j] - lo), c);
+      for (int j = 0; j < keys_per_lane<kW>(); ++j) {
+        if (k[j] >= kTombKey) continue;
+        const uint32_t v = k[j] - lo;
+        if (v < n)  // (a key below lo wraps above n)
+          atomicAdd(nx + v, c);
+        else
+          atomicOr(g.err, kErrInvalidId);
+      }
     });
   }
 }
 
+// Iterations up to which a run pushes: turning the edges around costs what two
+// to three pushes do.  Pushed / turned, microseconds: 4.1 M edges 142 / 354 at
+// one iteration, 399 / 425 at three, 530 / 459 at four; 1 M edges (weighted)
+// 79 / 191, 216 / 213, 282 / 230; 20,000 edges 41 / 84, 109 / 108, 134 / 120.
+constexpr uint32_t kPrrPushIters = 3;
 constexpr uint32_t kPrrChunk = 512;  // pairs per warp of the gather
 constexpr uint32_t kPrrBatch = 12;   // iterations issued between two reads of the deltas
 constexpr uint32_t kPrrSteps = 4;    // 32-pair steps whose loads are in flight together
@@ -416,23 +429,27 @@ mk_status mk_pagerank_range_run(mk_pagerank_range *p, uint32_t v_begin, uint32_t
   uint32_t it = 0;
   double delta = 0.0;
   unsigned long long E = 0;
-  const mk_status turned = prr_turn(p, v_begin, n, b0, nb, s, &E);
-  if (turned == MK_OK) {
+  bool push = max_iter <= kPrrPushIters;
+  if (!push) {
+    const mk_status turned = prr_turn(p, v_begin, n, b0, nb, s, &E);
+    push = turned == MK_ERR_OOM;  // the pairs do not fit beside what the process holds
+    if (push)
+      (void)cudaGetLastError();
+    else
+      MK_CHECK(turned);
+  }
+  if (!push) {
     MK_CHECK(prr_gather_solve(p, v_begin, n, E, d, 0.5 * tol, max_iter, s, &it, &delta));
-  } else if (turned != MK_ERR_OOM) {
-    return turned;
   } else {
-    // the pairs do not fit beside what the process holds: push from the slabs
-    (void)cudaGetLastError();
     k_prr_fill<<<fb, 256, 0, s>>>(pr, n, 1.0 / n);
     while (it < max_iter) {
       MK_CUDA(cudaMemsetAsync(p->acc, 0, 16, s));
       k_prr_dangling<<<fb, 256, 0, s>>>(pr, g->deg + v_begin, n, p->acc);
       k_prr_base<<<fb, 256, 0, s>>>(nx, n, p->acc, d);
       if (g->weighted)
-        k_prr_push<true><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
+        k_prr_push<true><<<gb, 256, 0, s>>>(v, v_begin, n, b0, nb, pr, nx, d);
       else
-        k_prr_push<false><<<gb, 256, 0, s>>>(v, v_begin, b0, nb, pr, nx, d);
+        k_prr_push<false><<<gb, 256, 0, s>>>(v, v_begin, n, b0, nb, pr, nx, d);
       k_prr_delta<<<fb, 256, 0, s>>>(pr, nx, n, p->acc);
       MK_CUDA(cudaGetLastError());
       MK_CUDA(cudaMemcpyAsync(&delta, p->acc + 1, 8, cudaMemcpyDeviceToHost, s));
