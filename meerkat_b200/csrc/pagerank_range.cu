@@ -204,22 +204,23 @@ __global__ void __launch_bounds__(256)
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
   for (uint64_t e0 = warp * kPrrChunk; e0 < E; e0 += nwarps * kPrrChunk) {
-    const uint64_t e1 = e0 + kPrrChunk < E ? e0 + kPrrChunk : E;
+    const uint32_t len = E - e0 < kPrrChunk ? (uint32_t)(E - e0) : kPrrChunk;
+    const uint2 *__restrict__ chunk = pairs + e0;
     uint32_t ckey = kEmptyKey;  // target whose run is open, and its sum so far
     double cval = 0.0;
-    for (uint64_t s0 = e0; s0 < e1; s0 += 32u * kPrrSteps) {
+    for (uint32_t s0 = 0; s0 < len; s0 += 32u * kPrrSteps) {
       uint2 p[kPrrSteps];
       double val[kPrrSteps];
 #pragma unroll
       for (uint32_t r = 0; r < kPrrSteps; ++r) {
-        const uint64_t e = s0 + 32u * r + lane;
-        p[r] = e < e1 ? __ldg(pairs + e) : make_uint2(0u, kEmptyKey);
+        const uint32_t e = s0 + 32u * r + lane;
+        p[r] = e < len ? __ldg(chunk + e) : make_uint2(0u, kEmptyKey);
       }
 #pragma unroll
       for (uint32_t r = 0; r < kPrrSteps; ++r) val[r] = p[r].y != kEmptyKey ? __ldg(c + p[r].x) : 0.0;
 #pragma unroll
       for (uint32_t r = 0; r < kPrrSteps; ++r) {
-        if (s0 + 32u * r >= e1) break;
+        if (s0 + 32u * r >= len) break;
         const uint32_t key = p[r].y;  // kEmptyKey: no edge here, val 0
         double v = val[r];
         if (lane == 0) {
