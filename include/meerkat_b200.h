@@ -352,7 +352,9 @@ mk_status mk_pagerank_destroy(mk_pagerank *p);
  * FP64 accumulation: no reverse graph needed.  A run turns the member's live
  * edges around in scratch (8 bytes per edge, kept by the handle; runs of at
  * most three iterations, and those that it does not fit for, push straight
- * from the slabs).  Same formula,
+ * from the slabs).  create sizes the scratch for the graph as it is; a run on
+ * a member that has grown past it grows it (which waits for the device).
+ * Same formula,
  * start and stopping rule as above with N = v_end - v_begin; out-degrees are
  * the graph's live degrees.  The range must be closed under out-edges, and
  * its edges must not change during the run (order updates before it or after
@@ -364,6 +366,11 @@ mk_status mk_pagerank_range_create(mk_graph *g, uint32_t max_vertices,
 mk_status mk_pagerank_range_run(mk_pagerank_range *p, uint32_t v_begin, uint32_t v_end,
                                 float damping, float tol, uint32_t max_iter,
                                 void *stream, float *ms_out);
+/* Sizes the turned edges' scratch for members of up to max_edges live edges
+ * (to the next power of two; blocking) and keeps it there: a run on a member
+ * with more pushes from the slabs instead of growing it.  0 (the state after
+ * create) lets it grow. */
+mk_status mk_pagerank_range_reserve(mk_pagerank_range *p, uint64_t max_edges);
 /* The last run's v_end - v_begin values (host). */
 mk_status mk_pagerank_range_values(mk_pagerank_range *p, float *h_out);
 mk_status mk_pagerank_range_stats(mk_pagerank_range *p, uint32_t *h_iters, float *h_delta);

@@ -486,6 +486,12 @@ class PageRankRange(_Timed):
         except Exception:
             pass
 
+    def reserve(self, max_edges: int) -> None:
+        """Sizes the scratch for members of up to max_edges live edges and
+        keeps it there (a run on a member with more pushes from the slabs);
+        0 lets runs grow it."""
+        check(lib().mk_pagerank_range_reserve(self._h, int(max_edges)), "mk_pagerank_range_reserve")
+
     def Run(self, v_begin: int, v_end: int, damping: float = 0.85, tol: float = 1e-6,
             max_iter: int = 200, stream=None, timed=True):
         self._n = int(v_end) - int(v_begin)

@@ -97,6 +97,7 @@ SIGNATURES = [
     ("mk_pagerank_range_create", _S, [vp, C.c_uint32, C.POINTER(vp)]),
     ("mk_pagerank_range_run", _S, [vp, C.c_uint32, C.c_uint32, C.c_float, C.c_float, C.c_uint32,
                                    vp, f32p]),
+    ("mk_pagerank_range_reserve", _S, [vp, C.c_uint64]),
     ("mk_pagerank_range_values", _S, [vp, vp]),
     ("mk_pagerank_range_stats", _S, [vp, u32p, f32p]),
     ("mk_pagerank_range_destroy", _S, [vp]),

@@ -239,10 +239,19 @@ class GraphServer:
         # (a later growth would synchronise the device mid-run)
         edges = [int(self.G.count_edges(lo, hi)) for lo, hi in ranges]
         big = int(np.argmax(edges))
-        # the range PageRank's turned edges and per-vertex words (its buffers
-        # grow in powers of two); it pushes from the slabs where they do not fit
+        # the range PageRank's per-vertex words (sized when it is created) and
+        # its turned edges, in powers of two: room for one more update of the
+        # largest member where the budget allows it beside the triangle counts,
+        # fixed here; a member that outgrows it is pushed from the slabs
         pow2 = lambda n: 1 << max(10, (int(n) - 1).bit_length())  # noqa: E731
-        self.resident += 8 * pow2(max(edges)) + 20 * pow2(sizes.max())
+        self.resident += 20 * pow2(sizes.max())
+        left = self.budget - self.resident - max(
+            TC_BYTES_PER_EDGE * e + TC_BYTES_PER_VERTEX * int(n) for e, n in zip(edges, sizes))
+        pairs = next((p for p in (pow2(max(edges) + int(max_update)), pow2(max(edges))) if 8 * p <= left),
+                     pow2(1))
+        self.prr.reserve(pairs)
+        self.pagerank_edges = pairs
+        self.resident += 8 * pairs
         warm = Request(rid=-1, graph=big, kind=TC_Q, arrival=0.0)
         self.run_heavy(warm, self.heavy)
         if warm.status != "ok":

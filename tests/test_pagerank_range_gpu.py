@@ -85,3 +85,38 @@ def test_range_pagerank_reports_an_edge_that_leaves_the_range(weighted, iters):
     assert np.isfinite(prr.Values()).all()
     with pytest.raises(mk.MeerkatError, match="vertex id out of range"):
         gs.graph.sync()
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def test_range_pagerank_scratch_is_sized_at_creation():
+    """No run on a member that has not grown allocates; a fixed scratch stays
+    as it is when the member outgrows it, with the same ranks."""
+    rng = np.random.default_rng(6)
+    key = np.unique(rng.integers(0, N * N, 700000))
+    s, d = key // N, key % N
+    s, d = s[s != d], d[s != d]
+    gs = _member(s, d, False)
+    prr = mk.PageRankRange(gs.graph, N)
+
+    def run(reserve=None):
+        if reserve is not None:
+            prr.reserve(reserve)
+        before = _free()
+        prr.Run(LEAD, LEAD + N, 0.85, 1e-30, 13)
+        assert _free() == before, reserve
+        err = np.abs(prr.Values().astype(np.float64) - _reference(s, d, 13, 0.85)).sum()
+        assert err <= 2.0 ** -24 + 1e-12, reserve
+
+    run()
+    run(len(s))
+    run(2000)  # far below the member: pushed from the slabs
+    prr.reserve(0)
+    free = _free()
+    prr.Run(LEAD, LEAD + N, 0.85, 1e-30, 13)
+    assert _free() < free  # grown again
+    assert gs.graph.sync() == 0

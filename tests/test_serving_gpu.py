@@ -120,6 +120,49 @@ def test_inserts_beyond_the_slab_pool_are_refused_not_failed():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("roomy", [True, False])
+def test_pagerank_scratch_stays_within_what_the_server_accounts_for(roomy):
+    """PageRank requests allocate nothing once the server stands, on the
+    member with the most vertices and on one that has grown past the scratch
+    (then pushed from the slabs), and their answers stay the oracle's."""
+    import torch
+    gs, edges, wl = make_server(17)
+    nv, voff = wl.num_vertices, gs.offsets.astype(np.int64)
+    budget = 1 << 40
+    if not roomy:  # what stands and the largest triangle count's scratch, no more
+        twin = make_server(17)[0]
+        probe = S.GraphServer(twin, budget_bytes=budget, max_update=1000)
+        tc = max(S.TC_BYTES_PER_EDGE * twin.graph.count_edges(voff[m], voff[m + 1])
+                 + S.TC_BYTES_PER_VERTEX * int(nv[m]) for m in range(len(nv)))
+        budget = probe.resident - 8 * probe.pagerank_edges + tc + 8 * 1024
+        probe.close()
+    srv = S.GraphServer(gs, budget_bytes=budget, record=True, max_update=1000)
+    assert srv.resident <= budget
+    assert srv.pagerank_edges >= wl.num_edges.max() if roomy else srv.pagerank_edges == 1024
+    g = int(np.argmax(nv))
+    Os = OracleGraph(int(nv[g]))
+    own = (h(edges[0]) >= voff[g]) & (h(edges[0]) < voff[g + 1])
+    Os.insert((h(edges[0])[own] - voff[g]).astype(np.uint32), (h(edges[1])[own] - voff[g]).astype(np.uint32))
+    rng = np.random.default_rng(3)
+    for grow in (0, 40000):
+        if grow:
+            u = rng.integers(0, nv[g], grow)
+            v = (u + 1 + rng.integers(0, nv[g] - 1, grow)) % nv[g]
+            td = lambda a: torch.from_numpy(a.astype(np.int32)).cuda()  # noqa: E731
+            gs.graph.InsertEdges(td(u + voff[g]), td(v + voff[g]), vals=td(np.ones(grow)))
+            Os.insert(u.astype(np.uint32), v.astype(np.uint32))
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        r = S.Request(rid=0, graph=g, kind=S.PAGERANK_Q, arrival=0.0)
+        srv.run_heavy(r, srv.heavy)
+        torch.cuda.synchronize()
+        assert torch.cuda.mem_get_info()[0] == free
+        assert r.status == "ok"
+        assert np.abs(r.result.astype(np.float64) - Os.pagerank(0.85, 1e-14)[0]).sum() <= PR_L1_TOL
+    srv.close()
+
+
+@pytest.mark.gpu
 def test_triangle_counts_beyond_the_budget_are_refused():
     seed = 6
     gs, edges, wl = make_server(seed)
