@@ -1332,7 +1332,9 @@ static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, 
   a.delta = g->tuning.sssp_delta;
   a.rg = t->rev ? t->rev->view() : GraphView{};
   if (!t->rev) a.rg.V = 0;
-  a.pull_items = (t->rev && g->tuning.pull_permille)
+  // a pulled level would neither keep the closed ranges' edges inside them nor
+  // see the ones that leave them (it stops at the first parent)
+  a.pull_items = (t->rev && g->tuning.pull_permille && !a.nclosed)
                      ? (uint32_t)std::max<uint64_t>(1, (uint64_t)g->V * g->tuning.pull_permille / 1000)
                      : 0u;
   a.recompute_inv = g->tuning.recompute_permille
@@ -1520,7 +1522,8 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   std::vector<uint32_t> small_ids, large_src;
   std::vector<std::pair<uint32_t, uint32_t>> spans;
   std::vector<std::pair<uint32_t, uint32_t>> closed;  // small enough, but heavy
-  uint64_t all = 0;  // buckets of all ranges
+  uint64_t all = 0;     // buckets of all ranges
+  uint32_t widest = 0;  // vertices of the widest
   for (uint32_t r = 0; r < nranges; ++r) {
     const uint32_t b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
     if (b >= e || e > g->V) return fail(MK_ERR_INVALID, std::string(what) + ": bad vertex range");
@@ -1528,13 +1531,18 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
       return fail(MK_ERR_INVALID, std::string(what) + ": source outside its range");
     spans.emplace_back(b, e);
     all += g->h_boff[e] - g->h_boff[b];
+    widest = std::max(widest, e - b);
   }
   // A range goes to the device-wide kernel when it is too large for shared
   // memory, or holds more than twice an SM's share of all buckets (and
   // enough of them to fill the device): its one CTA would still be walking it
   // when the other SMs are done.  Of 256 members of 1,024 to 65,535 vertices
   // (19 M edges) the largest held 8 shares and took the whole 2.3 ms.
-  const uint64_t heavy = std::max<uint64_t>(2 * all / (uint64_t)device_sm_count(g->device), kHeavyBuckets);
+  // Beside ranges too large for shared memory whose levels may be pulled, it
+  // stays with its CTA: with it the launch could not pull (trav_issue).
+  const uint64_t heavy = t->rev && g->tuning.pull_permille && widest > kMemLocalMax
+                             ? ~0ull
+                             : std::max<uint64_t>(2 * all / (uint64_t)device_sm_count(g->device), kHeavyBuckets);
   for (uint32_t r = 0; r < nranges; ++r) {
     const uint32_t b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
     if (e - b <= kMemLocalMax && g->h_boff[e] - g->h_boff[b] <= heavy) {

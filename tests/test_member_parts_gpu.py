@@ -53,6 +53,46 @@ def test_wcc_of_members_split_into_parts(kind, weighted):
     assert gs.graph.sync() == 0
 
 
+@pytest.mark.parametrize("extra", [[], [70000]])
+def test_members_that_outweigh_the_others_are_not_pulled(extra):
+    """With a reverse graph and pull levels on, an edge that leaves a heavy
+    member is skipped and reported all the same, with and without a member
+    too large for shared memory beside it."""
+    rng = np.random.default_rng(29)
+    sizes = [1500, 60001] + extra + [1100] * 20
+    gs = mk.GraphSet(sizes)
+    off = gs.offsets.astype(np.int64)
+    mem = [_edges("random", n, rng) for n in sizes]
+    s = np.concatenate([m[0] + off[i] for i, m in enumerate(mem)])
+    d = np.concatenate([m[1] + off[i] for i, m in enumerate(mem)])
+    src = [int(m[0][0]) for m in mem]
+    want = []
+    for i, (ms, md) in enumerate(mem):
+        O = OracleGraph(sizes[i])
+        O.insert(ms, md)
+        want.append(O.bfs(src[i]))
+    lost = int(np.flatnonzero(want[0] == want[0].max())[-1])  # a vertex its member does not reach
+    assert want[0][lost] > sizes[0]
+    reached = want[1] <= sizes[1]
+    wide = np.argmax(np.bincount(want[1][reached]))  # the level with the most vertices: a pulled one
+    s = np.append(s, off[1] + np.flatnonzero(want[1] == wide)[0])
+    d = np.append(d, off[0] + lost)
+    rev = mk.DynamicGraph(int(off[-1]), reverse=True)
+    gs.graph.InsertEdges(to_dev(s), to_dev(d))
+    rev.InsertEdges(to_dev(s), to_dev(d))
+    assert gs.graph.sync() == 0 and rev.sync() == 0
+    gs.graph.set_tuning(pull_permille=1)
+    bfs = mk.BFS(gs.graph, [int(off[i]) + src[i] for i in range(len(sizes))])
+    bfs.set_reverse(rev)
+    bfs.PrepareMembers([(int(off[i]), int(off[i + 1])) for i in range(len(sizes))])
+    bfs.StaticMembers()
+    dist = bfs.Distances()
+    for i in range(len(sizes)):
+        np.testing.assert_array_equal(dist[off[i]:off[i + 1]], want[i])
+    with pytest.raises(mk.MeerkatError, match="vertex id out of range"):
+        gs.graph.sync()
+
+
 @pytest.mark.parametrize("weighted", [False, True])
 def test_bfs_of_members_that_outweigh_the_others(weighted):
     """One member holds most buckets, so it goes through the device-wide
