@@ -274,7 +274,8 @@ mk_status mk_traversal_static(mk_traversal *t, void *stream, float *ms_out);
  * on `stream`, so it can be captured into a CUDA graph.  A range of at most
  * 65,535 vertices is solved by one CTA with its BFS state in shared memory,
  * unless it holds more than two SMs' share of all ranges' buckets; such and
- * larger ones by the device-wide kernel.  The distances of every vertex are
+ * larger ones by the device-wide kernel, which gives a range of at most 65,535
+ * vertices back to a CTA after 20 levels.  The distances of every vertex are
  * those mk_traversal_static gives and the parents form a valid BFS tree
  * (parents are not unique: of several equal-distance parents, the device-wide
  * kernel keeps the first to arrive, the member kernel the smallest id); an

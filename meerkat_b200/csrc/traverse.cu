@@ -96,6 +96,7 @@ struct TravArgs {
   // reported as MK_DEVERR_INVALID_ID, as the member kernel does)
   const uint2 *closed;
   uint32_t nclosed;
+  uint32_t *left;           // word per closed range: set when its walk was given up (kWideLevels)
   uint32_t chunk;           // buckets per frontier work item
   uint32_t mode;
   uint32_t delta;           // near-far SSSP step (0: the threshold doubles)
@@ -123,6 +124,13 @@ constexpr uint32_t kWarpFlush = 96;    // vertices from which it is emptied betw
 constexpr uint32_t kFarQueue = 160;    // the same for the far list (SSSP)
 constexpr uint32_t kFarFlush = 80;
 constexpr uint32_t kHeavyBuckets = 32768;  // a member below this never goes device-wide for its buckets
+// Levels after which the device-wide walk of such a member is given up: its
+// CTA then walks it after all.  A level costs 6 us device-wide and 1.5 us in a
+// CTA, so many thin levels are the CTA's: 255 x 255 grid 1.81 ms in a CTA,
+// 3.39 device-wide, 1.94 given up; a path of 40,000 vertices 60, 240 and 63
+// ms.  Random and R-MAT members of 4 to 64 edges a vertex are through by then
+// (device-wide 0.1 ms, in a CTA 0.4 to 1.3).
+constexpr uint32_t kWideLevels = 20;
 constexpr uint32_t kDefaultChunk = 4;  // buckets per frontier work item
 
 __host__ __device__ __forceinline__ unsigned long long item(uint32_t v, uint32_t chunk) {
@@ -472,8 +480,8 @@ __device__ __forceinline__ void visit_slabs4(const TravArgs &a, const Lanes &L, 
 }
 
 // The closed range of TravArgs that holds u, as its first vertex and size
-// (everything when none does).
-__device__ __forceinline__ void closed_range(const TravArgs &a, uint32_t u, uint32_t &lo, uint32_t &span) {
+// (everything when none does); returns its index (nclosed: none).
+__device__ __forceinline__ uint32_t closed_range(const TravArgs &a, uint32_t u, uint32_t &lo, uint32_t &span) {
   lo = 0u;
   span = kTombKey;
   uint32_t l = 0, h = a.nclosed;
@@ -487,9 +495,10 @@ __device__ __forceinline__ void closed_range(const TravArgs &a, uint32_t u, uint
     } else {
       lo = r.x;
       span = r.y - r.x;
-      return;
+      return m;
     }
   }
+  return a.nclosed;
 }
 
 // Bucket range of a work item.
@@ -1029,7 +1038,12 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
           item_range(a.g, now, a.chunk, u, b0, b1);
           if (!kUseW && a.vis) {
             uint32_t lo = 0u, span = kTombKey;
-            if (kClosed) closed_range(a, u, lo, span);
+            uint32_t m = 0;
+            if (kClosed) m = closed_range(a, u, lo, span);
+            if (kClosed && lv >= kWideLevels && m < a.nclosed) {
+              a.left[m] = 1u;  // not expanded: no later level of this range
+              b1 = b0;
+            }
             expand_range(a, L, b0, b1, [&](const uint4 (&q)[4], uint32_t nq) {
               visit_slabs4<kW, kClosed>(a, L, Q, q, nq, u, lo, span, lv, nxt, nsz);
             });
@@ -1103,11 +1117,14 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
 // counter, largest first.  rng[r] = (first vertex, end vertex, first bucket,
 // end bucket) of a range of at most kMemLocalMax vertices, src[r] its source
 // (global id).  items holds one word per bucket of the graph, found one per
-// vertex.  dist must already hold INFINF.
+// vertex.  dist must already hold INFINF, or for the first nwide ranges what
+// the device-wide kernel found: one that it gave up (left) is walked from the
+// start here, to the same levels.
 template <bool kW>
 __global__ void __launch_bounds__(kMemThreads, 1)
     k_bfs_members(GraphView g, const uint4 *__restrict__ rng, const uint32_t *__restrict__ src,
-                  uint32_t nr, uint32_t *counter, unsigned long long *__restrict__ dist,
+                  uint32_t nr, uint32_t *counter, const uint32_t *__restrict__ left, uint32_t nwide,
+                  unsigned long long *__restrict__ dist,
                   uint32_t *__restrict__ items, uint32_t *__restrict__ found, uint32_t *err) {
   extern __shared__ uint32_t smem[];
   __shared__ uint32_t s_range, s_nfound, s_nitems;
@@ -1117,6 +1134,10 @@ __global__ void __launch_bounds__(kMemThreads, 1)
     __syncthreads();
     const uint32_t r = s_range;
     if (r >= nr) break;
+    if (r < nwide && !left[r]) {
+      __syncthreads();  // before s_range is written again
+      continue;
+    }
     bfs_member<kW, false>(g, L, rng[r], src[r], dist, items, found, err, smem, s_nfound, s_nitems);
   }
 }
@@ -1150,13 +1171,17 @@ struct mk_traversal {
   uint32_t *tcand0 = nullptr, *tcand1 = nullptr, *tpar = nullptr;
   size_t rcap = 0;  // re-seed / support item capacity
   std::vector<uint32_t> h_sources;
-  // prepared member table (BFS): counter word, uint4 (lo, hi, b0, b1) per
-  // small range (most buckets first), their sources, then the sources whose
-  // range is too large for shared memory
+  // prepared member table (BFS): counter word, a word per closed range (given
+  // up; zeroed with the counter before every launch) up to a multiple of 4
+  // words, uint4 (lo, hi, b0, b1) per small range (the closed ones by vertex,
+  // then the others, most buckets first), their sources, then the sources of
+  // the device-wide kernel, then (lo, hi) of the closed ranges: small ones
+  // that go device-wide first, for their buckets
   DevBuf<uint32_t> members;
   uint32_t n_small = 0, n_large = 0, small_max = 0;
-  const uint2 *d_closed = nullptr;  // in members: the ranges that went device-wide for their buckets
+  const uint2 *d_closed = nullptr;  // in members
   uint32_t n_closed = 0;
+  size_t member_head() const { return (1 + (size_t)n_closed + 3) / 4 * 4; }
   int small_grid = 0;
   bool members_prepared = false;
   PinnedRing staging;  // stream-ordered source uploads
@@ -1328,6 +1353,7 @@ static mk_status trav_issue(mk_traversal *t, uint32_t mode, const uint32_t *bs, 
   a.nsources = srcs ? nsrc : t->nsources;
   a.closed = srcs ? t->d_closed : nullptr;
   a.nclosed = srcs ? t->n_closed : 0u;
+  a.left = srcs ? t->members.ptr + 1 : nullptr;
   a.chunk = g->tuning.frontier_chunk ? g->tuning.frontier_chunk : kDefaultChunk;
   a.delta = g->tuning.sssp_delta;
   a.rg = t->rev ? t->rev->view() : GraphView{};
@@ -1521,7 +1547,7 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   mk_graph *g = t->g;
   std::vector<uint32_t> small_ids, large_src;
   std::vector<std::pair<uint32_t, uint32_t>> spans;
-  std::vector<std::pair<uint32_t, uint32_t>> closed;  // small enough, but heavy
+  std::vector<uint32_t> closed;  // small enough, but heavy
   uint64_t all = 0;     // buckets of all ranges
   uint32_t widest = 0;  // vertices of the widest
   for (uint32_t r = 0; r < nranges; ++r) {
@@ -1549,10 +1575,11 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
       small_ids.push_back(r);
     } else {
       large_src.push_back(t->h_sources[r]);
-      if (e - b <= kMemLocalMax) closed.emplace_back(b, e);
+      if (e - b <= kMemLocalMax) closed.push_back(r);
     }
   }
-  std::sort(closed.begin(), closed.end());
+  std::sort(closed.begin(), closed.end(),
+            [&](uint32_t a, uint32_t b) { return h_vertex_ranges[2 * a] < h_vertex_ranges[2 * b]; });
   std::sort(spans.begin(), spans.end());
   for (size_t i = 1; i < spans.size(); ++i)
     if (spans[i].first < spans[i - 1].second)
@@ -1565,14 +1592,16 @@ mk_status mk_bfs_prepare_members(mk_traversal *t, const uint32_t *h_vertex_range
   // differ eightfold between members
   std::stable_sort(small_ids.begin(), small_ids.end(),
                    [&](uint32_t a, uint32_t b) { return buckets(a) > buckets(b); });
+  small_ids.insert(small_ids.begin(), closed.begin(), closed.end());
   const size_t ns = small_ids.size(), nl = large_src.size();
   const size_t nc = closed.size();
-  const size_t lists = (4 + 5 * ns + nl + 1) / 2 * 2;  // the pairs behind start on 8 bytes
+  const size_t head = (1 + nc + 3) / 4 * 4;
+  const size_t lists = (head + 5 * ns + nl + 1) / 2 * 2;  // the pairs behind start on 8 bytes
   std::vector<uint32_t> host(lists + 2 * nc, 0u);
-  uint32_t *tab = host.data() + 4, *ssrc = tab + 4 * ns, *lsrc = ssrc + ns;
+  uint32_t *tab = host.data() + head, *ssrc = tab + 4 * ns, *lsrc = ssrc + ns;
   for (size_t i = 0; i < nc; ++i) {
-    host[lists + 2 * i] = closed[i].first;
-    host[lists + 2 * i + 1] = closed[i].second;
+    host[lists + 2 * i] = h_vertex_ranges[2 * closed[i]];
+    host[lists + 2 * i + 1] = h_vertex_ranges[2 * closed[i] + 1];
   }
   for (size_t i = 0; i < ns; ++i) {
     const uint32_t r = small_ids[i], b = h_vertex_ranges[2 * r], e = h_vertex_ranges[2 * r + 1];
@@ -1625,11 +1654,12 @@ mk_status trav_static_members(mk_traversal *t, void *stream, float *ms_out, cuda
   MK_CHECK(t->timer.start(s, ms_out != nullptr));
   const uint32_t ns = t->n_small, nl = t->n_large;
   uint32_t *counter = t->members.ptr;
-  const uint4 *tab = reinterpret_cast<const uint4 *>(counter + 4);
-  const uint32_t *ssrc = counter + 4 + 4 * (size_t)ns, *lsrc = ssrc + ns;
+  const uint4 *tab = reinterpret_cast<const uint4 *>(counter + t->member_head());
+  const uint32_t *ssrc = counter + t->member_head() + 4 * (size_t)ns, *lsrc = ssrc + ns;
+  if (ns) MK_CUDA(cudaMemsetAsync(counter, 0, (1 + (size_t)t->n_closed) * 4, s));
   if (nl) {
-    // ranges too large for shared memory: the device-wide kernel from their
-    // sources (it also resets every distance)
+    // ranges too large for shared memory, and heavy ones: the device-wide
+    // kernel from their sources (it also resets every distance)
     MK_CHECK(trav_issue(t, kStatic, nullptr, nullptr, 0, s, lsrc, nl));
   } else {
     trav_begin(t, true, false, false, s);
@@ -1637,14 +1667,15 @@ mk_status trav_static_members(mk_traversal *t, void *stream, float *ms_out, cuda
   if (wide_done) MK_CUDA(cudaEventRecord(wide_done, s));
   if (ns) {
     const size_t smem = bfs_member_smem(t->small_max);
-    MK_CUDA(cudaMemsetAsync(counter, 0, 4, s));
     uint32_t *items = reinterpret_cast<uint32_t *>(t->fr0);
     if (g->weighted)
-      k_bfs_members<true><<<t->small_grid, kMemThreads, smem, s>>>(g->view(), tab, ssrc, ns, counter, t->dist,
-                                                                   items, t->inv_list, g->err_word());
+      k_bfs_members<true><<<t->small_grid, kMemThreads, smem, s>>>(g->view(), tab, ssrc, ns, counter, counter + 1,
+                                                                   t->n_closed, t->dist, items, t->inv_list,
+                                                                   g->err_word());
     else
-      k_bfs_members<false><<<t->small_grid, kMemThreads, smem, s>>>(g->view(), tab, ssrc, ns, counter, t->dist,
-                                                                    items, t->inv_list, g->err_word());
+      k_bfs_members<false><<<t->small_grid, kMemThreads, smem, s>>>(g->view(), tab, ssrc, ns, counter, counter + 1,
+                                                                    t->n_closed, t->dist, items, t->inv_list,
+                                                                    g->err_word());
     MK_CUDA(cudaGetLastError());
   }
   MK_CHECK(t->timer.stop(ms_out));

@@ -126,3 +126,43 @@ def test_bfs_of_members_that_outweigh_the_others(weighted):
     np.testing.assert_array_equal(bfs.Distances()[off[0]:off[1]], before)
     with pytest.raises(mk.MeerkatError, match="vertex id out of range"):
         gs.graph.sync()
+
+
+def _layers(depth, n, rng):
+    """A source and depth layers of its own, every vertex reached from the layer before."""
+    cut = np.concatenate([[0], np.linspace(1, n, depth + 1).astype(int)])
+    s = [rng.integers(cut[i], cut[i + 1], cut[i + 2] - cut[i + 1]) for i in range(depth)]
+    return np.concatenate(s).astype(np.uint32), np.arange(1, n, dtype=np.uint32)
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_bfs_of_heavy_members_with_many_levels(weighted):
+    """Heavy members whose walk ends just before, at and after the level where
+    the device-wide kernel gives a member up, one far beyond it, one shallow;
+    beside them a member too large for shared memory, as deep, and small ones."""
+    rng = np.random.default_rng(31)
+    depths = [18, 19, 20, 21, 22, 400]
+    mem = [_layers(k, 33000 + 7 * k, rng) for k in depths] + [_edges("random", 50000, rng)]
+    mem += [_layers(300, 70000, rng)] + [_edges("random", 700, rng) for _ in range(12)]
+    sizes = [33000 + 7 * k for k in depths] + [50000, 70000] + [700] * 12
+    gs = mk.GraphSet(sizes, weighted=weighted)
+    off = gs.offsets.astype(np.int64)
+    s = np.concatenate([m[0] + off[i] for i, m in enumerate(mem)])
+    d = np.concatenate([m[1] + off[i] for i, m in enumerate(mem)])
+    w = to_dev(np.ones(len(s), np.uint32)) if weighted else None
+    gs.graph.InsertEdges(to_dev(s), to_dev(d), vals=w)
+    order = rng.permutation(len(sizes))
+    src = [int(m[0][0]) for m in mem]
+    bfs = mk.BFS(gs.graph, [int(off[i]) + src[i] for i in order])
+    bfs.PrepareMembers([(int(off[i]), int(off[i + 1])) for i in order])
+    want = []
+    for i, (ms, md) in enumerate(mem):
+        O = OracleGraph(sizes[i])
+        O.insert(ms, md)
+        want.append(O.bfs(src[i]))
+    for _ in range(2):
+        bfs.StaticMembers()
+        dist = bfs.Distances()
+        for i in range(len(sizes)):
+            np.testing.assert_array_equal(dist[off[i]:off[i + 1]], want[i])
+    assert gs.graph.sync() == 0
