@@ -574,8 +574,8 @@ mk_status mk_gen_set_batches(const uint32_t *d_vertex_offsets, uint32_t num_grap
  * components) or MK_QUERY_NONE.  create uploads the query tables (blocking).
  * step applies one update batch covering any members (deletes, then inserts;
  * global vertex ids, device arrays; d_ins_w may be NULL) and then answers
- * every member's query: four launches (one more when a member outweighs the
- * others), all asynchronous, ordered on `stream` (the components run beside
+ * every member's query: four launches (one more when a BFS member outweighs
+ * the others), all asynchronous, ordered on `stream` (the components run beside
  * the BFS on a stream of the runner's own that joins it) and
  * allocation-free once mk_graph_reserve_batch has sized the batch scratch,
  * so a step can be captured into a CUDA graph.  A member's answers equal
@@ -604,8 +604,9 @@ mk_status mk_set_runner_step(mk_set_runner *r, const uint32_t *d_del_src,
  * keeps the four-launch step). */
 mk_status mk_set_runner_set_single(mk_set_runner *r, uint32_t on);
 /* Kernel launches one step issues: 1 in the one-launch form, else 2 plus
- * one per query kind present (members beyond one CTA's shared memory add the
- * device-wide kernels, not counted here). */
+ * one per query kind present, and one more when BFS members outweigh the
+ * others (members beyond one CTA's shared memory add the device-wide kernels,
+ * not counted here). */
 mk_status mk_set_runner_launches(mk_set_runner *r, uint32_t *h_launches);
 /* The runner's BFS and WCC handles (owned by the runner; NULL when no member
  * asks that query), for mk_traversal_distances / mk_wcc_labels. */

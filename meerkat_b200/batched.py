@@ -146,9 +146,12 @@ class BatchedRunner:
             return 1
         # kernels: delete, insert; BFS: 1 shared-memory kernel (plus 2
         # memsets) and the cooperative device-wide kernel when some member is
-        # larger than shared memory holds; WCC: 1 shared-memory kernel (plus 1
-        # memset), and 5 device-wide kernels for such members
-        bfs = (1 + (1 if self._bfs_large else 0)) if self.bfs is not None else 0
+        # larger than shared memory holds or outweighs the others (the C
+        # runner counts it for the latter); WCC: 1 shared-memory kernel (plus 1
+        # memset), and 5 device-wide kernels for the former
+        kinds = (self.bfs is not None) + (self.wcc is not None)
+        wide = self._bfs_large or self.runner.launches_per_step() > 2 + kinds
+        bfs = (1 + (1 if wide else 0)) if self.bfs is not None else 0
         wcc = (1 + (5 if self._wcc_large else 0)) if self.wcc is not None else 0
         return 2 + bfs + wcc
 

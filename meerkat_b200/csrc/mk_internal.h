@@ -130,6 +130,8 @@ struct TravMemberBufs {
   uint32_t *found;
 };
 mk_status trav_member_bufs(mk_traversal *t, TravMemberBufs *out);
+// Whether members that fit a CTA go through the device-wide kernel first.
+bool trav_heavy_members(const mk_traversal *t);
 // mk_bfs_static_members; wide_done (if given) is recorded behind the
 // device-wide part, before the member kernel.
 mk_status trav_static_members(mk_traversal *t, void *stream, float *ms_out, cudaEvent_t wide_done);

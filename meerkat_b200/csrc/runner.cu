@@ -6,10 +6,12 @@
 // algorithm object per process (src/BFS.cu:11-131); this is the path a C++
 // caller of the drop-in uses for thousands of small graphs.  Two forms:
 //
-//   sequence  four stream-ordered launches, those of the Python batched
-//             runner: one delete and one insert kernel over all members'
-//             batches, one shared-memory member BFS over the BFS members,
-//             one member WCC over the WCC members;
+//   sequence  those of the Python batched runner: one delete and one insert
+//             kernel over all members' batches, one shared-memory member BFS
+//             over the BFS members (behind a device-wide one for members
+//             that outweigh the others), and one member WCC over the WCC
+//             members beside it, on a stream of the runner's own that the
+//             caller's joins again;
 //   one launch  (mk_set_runner_set_single, every member of at most 65,535
 //             vertices) a cooperative kernel, one 1,024-thread CTA per SM,
 //             in three phases separated by bounded grid barriers: every
@@ -286,7 +288,8 @@ mk_status mk_set_runner_set_single(mk_set_runner *r, uint32_t on) {
 
 mk_status mk_set_runner_launches(mk_set_runner *r, uint32_t *h_launches) {
   if (!r || !h_launches) return fail(MK_ERR_INVALID, "mk_set_runner_launches: null argument");
-  *h_launches = r->single ? 1u : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u);
+  *h_launches = r->single ? 1u
+                          : 2u + (r->bfs ? 1u : 0u) + (r->wcc ? 1u : 0u) + (trav_heavy_members(r->bfs) ? 1u : 0u);
   return MK_OK;
 }
 

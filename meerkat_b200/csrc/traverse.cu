@@ -1421,6 +1421,8 @@ mk_status trav_member_bufs(mk_traversal *t, TravMemberBufs *out) {
   out->found = t->inv_list;
   return MK_OK;
 }
+
+bool trav_heavy_members(const mk_traversal *t) { return t && t->n_closed != 0; }
 }  // namespace mk
 
 extern "C" {

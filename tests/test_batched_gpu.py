@@ -161,6 +161,45 @@ def test_runner_step_matches_oracle(capture, weighted, single):
     gs.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("capture,weighted", [(False, False), (False, True), (True, False), (True, True)])
+def test_runner_step_with_members_that_outweigh_the_others(capture, weighted):
+    """A BFS and a WCC member hold most of the set, so the BFS member goes
+    device-wide first and the components run on the runner's own stream, in
+    several parts: answers and degrees equal the oracle's after each step,
+    issued directly or captured (fork and join included) and replayed, and the
+    launches of a step are counted with the device-wide one."""
+    import torch
+    nv = np.array([60000, 50000] + [900] * 20)
+    ne = np.concatenate([[480000, 600000], np.full(20, 5000)])
+    query = np.array([B.QUERY_BFS, B.QUERY_WCC] * 11, np.uint8)
+    spec = B.SetSpec(nv, ne, ne // 30, ne // 20, query, 15)
+    gs, _, oracles, voff = build(spec, "cuda:0", weighted=weighted)
+    bfs_members = np.flatnonzero(query == B.QUERY_BFS)
+    srcs = B.pick_sources(gs.graph.degrees(), voff, bfs_members, seed=5)
+    br = B.BatchedRunner(gs, query, srcs)
+    assert br.launches_per_step() == br.runner.launches_per_step() == 5
+    gs.graph.reserve_batch(int(max(spec.inserts.sum(), spec.deletes.sum())))
+    src_of = dict(zip(bfs_members.tolist(), srcs.tolist()))
+    for step in range(3):
+        batch = gs.gen_batches(spec.deletes, spec.inserts, seed=300 + step, weights=weighted)
+        if capture:
+            s = torch.cuda.Stream()
+            s.wait_stream(torch.cuda.current_stream())
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                br.step(batch, stream=s)
+            with torch.cuda.stream(s):
+                g.replay()
+            torch.cuda.synchronize()
+            del g
+        else:
+            br.step(batch)
+        check_step(spec, batch, voff, oracles, gs, br, src_of)
+    br.close()
+    gs.close()
+
+
 def test_spec_is_seeded_and_in_range():
     a = B.make_spec(500, seed=5)
     b = B.make_spec(500, seed=5)
