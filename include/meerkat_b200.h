@@ -184,6 +184,7 @@ mk_status mk_graph_reserve_batch(mk_graph *g, uint32_t n);
 /* Kernel choices of the update path (no counterpart in the reference, which
  * has a single insert/delete kernel).  The autotuner in
  * meerkat_b200/autotune.py measures the variants on live batches. */
+#define MK_SSSP_NO_SPLIT 0xFFFFFFFFu
 typedef struct mk_tuning {
   uint32_t update_kernel;        /* 0 = warp-staged (TMA bulk copies into shared
                                     memory), 1 = one lane per edge,
@@ -196,7 +197,8 @@ typedef struct mk_tuning {
                                     until the near frontier drains, then the
                                     threshold moves on by this much; 0 =
                                     automatic (it doubles; below a million
-                                    buckets no split)                          */
+                                    buckets no split), MK_SSSP_NO_SPLIT = off
+                                    (plain level-synchronous)                  */
   uint32_t recompute_permille;   /* decremental BFS/SSSP: once this share of
                                     the vertices (per mille) is invalidated,
                                     recompute from the sources instead of
