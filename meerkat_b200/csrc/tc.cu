@@ -181,7 +181,7 @@ __device__ __noinline__ uint32_t bucket_probe_on(const uint4 *set, uint32_t nb, 
   return 0u;
 }
 
-constexpr uint32_t kTcChunk = 32;  // partners per work item (one per lane)
+constexpr uint32_t kTcChunk = 32;  // partners per work item: one per lane
 constexpr int kTcSteps = 4;        // 32-entry probe steps with their loads in flight together
 
 // Length of every oriented list.
@@ -321,34 +321,32 @@ __global__ void __launch_bounds__(kTcWarps * 32)
     }
     const unsigned long long p0 = prow[u] + (unsigned long long)chunk * kTcChunk;
     const unsigned long long pe = prow[u + 1];
-    uint32_t c = 0;  // this item's triangles found by the lane (at most 32 lists of 2^32 / 32 entries)
-    for (unsigned long long pb = p0; pb < p0 + kTcChunk && pb < pe; pb += 32) {
-      const uint32_t m = pe - pb < 32 ? (uint32_t)(pe - pb) : 32u;
-      // one partner's list per lane, handed round below
-      unsigned long long ls = 0;
-      uint32_t ll = 0;
-      if (lane < m) {
-        const uint32_t x = pcol[pb + lane];
-        ls = orow[x];
-        ll = odeg[x];
-      }
-      for (uint32_t i = 0; i < m; ++i) {
-        const uint32_t *list = ocol + __shfl_sync(0xFFFFFFFFu, ls, i);
-        const uint32_t len = __shfl_sync(0xFFFFFFFFu, ll, i);
-        for (uint32_t x0 = lane; x0 - lane < len; x0 += 32u * kTcSteps) {
-          uint32_t key[kTcSteps];
-          // past the end: kTombKey, which no list and no set holds
+    const uint32_t m = pe - p0 < kTcChunk ? (uint32_t)(pe - p0) : kTcChunk;
+    uint32_t c = 0;  // this item's triangles found by the lane (at most kTcChunk times the set's 1,024 keys)
+    // one partner's list per lane, handed round below
+    unsigned long long ls = 0;
+    uint32_t ll = 0;
+    if (lane < m) {
+      const uint32_t x = pcol[p0 + lane];
+      ls = orow[x];
+      ll = odeg[x];
+    }
+    for (uint32_t i = 0; i < m; ++i) {
+      const uint32_t *list = ocol + __shfl_sync(0xFFFFFFFFu, ls, i);
+      const uint32_t len = __shfl_sync(0xFFFFFFFFu, ll, i);
+      for (uint32_t x0 = lane; x0 - lane < len; x0 += 32u * kTcSteps) {
+        uint32_t key[kTcSteps];
+        // past the end: kTombKey, which no list and no set holds
 #pragma unroll
-          for (int q = 0; q < kTcSteps; ++q) key[q] = x0 + 32u * q < len ? __ldg(list + x0 + 32u * q) : kTombKey;
+        for (int q = 0; q < kTcSteps; ++q) key[q] = x0 + 32u * q < len ? __ldg(list + x0 + 32u * q) : kTombKey;
 #pragma unroll
-          for (int q = 0; q < kTcSteps; ++q) {
-            const uint32_t h = bucket_slot(key[q], bshift);
-            const uint4 w = set[h];
-            if (w.x == key[q] || w.y == key[q] || w.z == key[q] || w.w == key[q])
-              ++c;
-            else if (w.w != kEmptyKey && key[q] != kTombKey)
-              c += bucket_probe_on(set, nb, h, key[q]);
-          }
+        for (int q = 0; q < kTcSteps; ++q) {
+          const uint32_t h = bucket_slot(key[q], bshift);
+          const uint4 w = set[h];
+          if (w.x == key[q] || w.y == key[q] || w.z == key[q] || w.w == key[q])
+            ++c;
+          else if (w.w != kEmptyKey && key[q] != kTombKey)
+            c += bucket_probe_on(set, nb, h, key[q]);
         }
       }
     }
@@ -650,7 +648,9 @@ struct mk_tc {
   Timer timer;
 };
 
-// Edges from which the static counts sort them by owner: the sort is seven
+// Edges from which the static counts sort them by owner (oriented ones of a
+// whole graph; of a member its directed ones, of which the host knows the
+// number, and which are up to twice the oriented): the sort is seven
 // more launches, which pay from about half a million edges (100,000 oriented
 // ones: 162 -> 205 us with it; a million: 423 -> 415 us; 7.5 million: 5.5 ->
 // 2.9 ms).

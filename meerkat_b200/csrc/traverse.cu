@@ -250,7 +250,6 @@ __device__ __forceinline__ unsigned long long ld_dist(const unsigned long long *
 // sends everything to the next level.  Far pushes gather in a queue per warp
 // as the near ones do, with the smallest distance pushed.
 constexpr uint32_t kNoFar = 0xFFFFFFFFu;
-constexpr uint32_t kFarShift = 0;
 // Buckets from which static SSSP without a step splits at all.  Below, a level
 // costs its fixed 8 us and not its work, and the phases run more levels:
 // 60,000 vertices, 600,000 edges R-MAT 433 us split, 311 us for the plain
@@ -321,7 +320,7 @@ __device__ __forceinline__ bool far_full(const NearFar &nf) {
 // every improvement expands at once, weights U[1, 1000]) in about twice the
 // levels; the number of phases is at most 32.
 __device__ __forceinline__ uint32_t next_threshold(uint32_t lo, uint32_t delta) {
-  const uint32_t step = delta ? delta : max(lo >> kFarShift, 1u);
+  const uint32_t step = delta ? delta : max(lo, 1u);
   return lo > kNoFar - step ? kNoFar : lo + step;
 }
 
@@ -524,8 +523,7 @@ __device__ __forceinline__ bool is_source(unsigned long long p, uint32_t v) {
 template <bool kRW>
 __device__ __forceinline__ void pull_level(const TravArgs &a, const Lanes &L, const WarpQueue &Q,
                                            uint32_t group, uint32_t ngroups, uint32_t lvl,
-                                           uint32_t stamp_next, unsigned long long *nxt,
-                                           uint32_t *nsz) {
+                                           unsigned long long *nxt, uint32_t *nsz) {
   const GraphView &rg = a.rg;
   for (uint32_t v = group; v < rg.V; v += ngroups) {
     unsigned long long pv = 0;
@@ -1017,9 +1015,9 @@ __global__ void __launch_bounds__(kTravBlock) k_traverse(TravArgs a) {
     if (n && !kUseW && a.mode == kStatic && a.pull_items && n >= a.pull_items) {
       // large BFS frontier: pull this level from the unvisited side
       if (a.rg.weighted)
-        pull_level<true>(a, L, Q, group, ngroups, lv, stamp_next, nxt, nsz);
+        pull_level<true>(a, L, Q, group, ngroups, lv, nxt, nsz);
       else
-        pull_level<false>(a, L, Q, group, ngroups, lv, stamp_next, nxt, nsz);
+        pull_level<false>(a, L, Q, group, ngroups, lv, nxt, nsz);
     } else if (n) {
       const NearFar nf = nearfar ? NearFar{thr, fb ? a.far1 : a.far0, ctl + kFarN0 + drain,
                                            ctl + kFarMin0 + drain, fq_s[kUseW ? threadIdx.x >> 5 : 0],
