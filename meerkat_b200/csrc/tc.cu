@@ -255,7 +255,7 @@ __global__ void k_tc_item_count(uint32_t V, const unsigned long long *__restrict
                                 uint32_t *big_max) {
   for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < V; u += gridDim.x * blockDim.x) {
     const uint32_t du = (uint32_t)(orow[u + 1] - orow[u]), np = (uint32_t)(prow[u + 1] - prow[u]);
-    odeg[u] = du;
+    if (odeg) odeg[u] = du;  // null: k_tc_odeg has written them
     uint32_t c = 0;
     if (du && np) {
       if (du > kTcSmallMax) {
@@ -740,8 +740,8 @@ static mk_status tc_count_oriented(mk_tc *t, uint32_t V, int device, TcOwners ow
   // work items (the orientation scratch is free again: ocnt >= V words,
   // bpos >= V + 1)
   const int vb = (int)std::min<uint64_t>((uint64_t)V / 256 + 1, (uint64_t)device_sm_count(device) * 8);
-  k_tc_item_count<<<vb, 256, 0, s>>>(V, t->orow.ptr, prow, own.odeg, t->ocnt.ptr, t->big_list.ptr, t->small,
-                                     t->small + 2);
+  k_tc_item_count<<<vb, 256, 0, s>>>(V, t->orow.ptr, prow, own.pcol ? nullptr : own.odeg, t->ocnt.ptr,
+                                     t->big_list.ptr, t->small, t->small + 2);
   MK_CHECK(scan_u32_to_u64(t->ocnt.ptr, t->bpos.ptr, V, t->tmp, s));
   unsigned long long nitems = 0;
   uint32_t hs[4] = {0, 0, 0, 0};  // [0] big vertices, [2] their largest oriented degree
