@@ -1076,7 +1076,7 @@ def grid_stress(side, nbatch, batch, rank, world, local):
     Gr.reserve_batch(batch)
     wcc.set_reverse(Gr)
     from meerkat_b200.autotune import SSSP_NO_SPLIT, tune_sssp_delta
-    nf = tune_sssp_delta(G, sssp, deltas=(0, 4096, 16384, 65536, SSSP_NO_SPLIT))
+    nf = tune_sssp_delta(G, sssp, deltas=(SSSP_NO_SPLIT, 0, 4096, 16384, 65536))
     # deletes aimed at the SSSP tree cut off large subtrees: recompute from the
     # centre once 0.5% of the vertices are invalidated instead of repairing
     G.set_tuning(recompute_permille=5)
@@ -1476,7 +1476,7 @@ def main():
         # the project tuner picks the static near-far step on this graph
         # (static calls are idempotent); the dynamic calls below keep it
         from meerkat_b200.autotune import SSSP_NO_SPLIT, tune_sssp_delta
-        nf = tune_sssp_delta(G, sssp, deltas=(0, 1000, 4000, 16000, SSSP_NO_SPLIT))
+        nf = tune_sssp_delta(G, sssp, deltas=(SSSP_NO_SPLIT, 0, 1000, 4000, 16000))
         algo["sssp_static_ms"] = min(t["static_ms"] for t in nf["trials"])
         algo["sssp_delta"] = nf["best"]
         algo["sssp_static_ms_plain"] = next(t["static_ms"] for t in nf["trials"] if t["sssp_delta"] == SSSP_NO_SPLIT)

@@ -118,7 +118,7 @@ def tune_frontier_chunk(G, traversal, chunks: Sequence[int] = CHUNKS, repeats: i
 # static SSSP near-far steps (0 = automatic: the threshold doubles on large
 # graphs; SSSP_NO_SPLIT, the header's MK_SSSP_NO_SPLIT: plain level-synchronous)
 SSSP_NO_SPLIT = 0xFFFFFFFF
-SSSP_DELTAS: Tuple[int, ...] = (0, 128, 512, 2048, 8192, SSSP_NO_SPLIT)
+SSSP_DELTAS: Tuple[int, ...] = (SSSP_NO_SPLIT, 0, 128, 512, 2048, 8192)
 
 
 def tune_sssp_delta(G, sssp, deltas: Sequence[int] = SSSP_DELTAS, repeats: int = 2) -> dict:

@@ -188,10 +188,10 @@ constexpr int kPrSteps = 4;         // 32-edge steps of the flat pass whose load
 // Segmented inclusive sum across the warp: each lane ends with the sum of its
 // run up to itself (a fixed tree order, the same in both forms).  kPos: tag
 // is the lane's position in its run, so no keys are shuffled, which frees the
-// pipe the gathers share (32 M edges: 3.86 -> 3.52 ms); else tag is the run's
-// key, whose compares wait on nothing before them: a solve of few edges is
-// bound by each warp's own latency (2.4 M edges: 0.86 against 0.89 ms,
-// 240,000: 0.55 against 0.60).
+// pipe the gathers share (32 M edges: 3.52 ms against 3.73 with keys); else tag
+// is the run's key, whose compares wait on nothing before them: a solve of few
+// edges is bound by each warp's own latency (2.4 M edges: 0.82 ms against 0.91
+// by position, 240,000: 0.53 against 0.59).
 template <bool kPos>
 __device__ __forceinline__ float seg_scan(float v, uint32_t tag, uint32_t lane) {
 #pragma unroll

@@ -263,8 +263,10 @@ __device__ __forceinline__ void link_bucket_skip(const GraphView &g, const Lanes
 // With `big` (k_uf_big_bits, which stand during the pass) an edge with both
 // ends in the big set is skipped on its key's bit alone: a bit is 32 times
 // denser than a parent word, so most tests hit L1, and on a graph with a
-// giant component 99 % of the edges end there (48 M edges: 805 us reading
-// every key's parent through L2, see the static passes for the rest).
+// giant component 99 % of the edges end there.  What bounded the pass before
+// was the instruction cache (the union inlined at every key), not these reads:
+// with the union in one function the bits take a static call on 48 M edges
+// from 780 to 764 us.
 template <bool kW>
 __global__ void k_uf_edges_skip(GraphView g, uint32_t *p, const uint32_t *sel_bits, uint32_t *err,
                                 unsigned long long *fe, const unsigned long long *skip_if = nullptr,
@@ -1013,9 +1015,10 @@ static mk_status wcc_link(mk_wcc *w, const uint32_t *sel, cudaStream_t s) {
   k_uf_compress<<<fg, 256, 0, s>>>(w->parent, g->V, sel);
   uint32_t *big = nullptr;
   // The whole graph: the big set's bits go where the next repair puts its own.
-  // Two small launches (about 15 us) that pay from about half a million
-  // buckets (500,000 vertices, 6 M edges: 267 -> 218 us; 360,000 grid
-  // vertices: 184 -> 200 us).
+  // Two small launches that pay from some hundred thousand buckets on (R-MAT,
+  // 12 edges a vertex, without / with them: 60,000 vertices 79-87 / 88 us,
+  // 200,000 147 / 143, 400,000 188 / 178, 500,000 225 / 212) and cost a grid
+  // their launches (360,000 vertices 184-210 / 195-220).
   if (!sel && g->num_buckets >= kBigBuckets) {
     big = w->aff_vertices;
     MK_CUDA(cudaMemsetAsync(w->fctl, 0, kFCtlWords * 8, s));

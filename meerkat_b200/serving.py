@@ -26,7 +26,8 @@ inserts still in flight, plus m would pass the slab pool's capacity, and is
 rejected when nothing in flight can change that (deletes never free slabs).
 Triangle counting's scratch grows to the largest member counted; a member
 whose scratch would take the resident set past the memory budget is
-rejected.
+rejected.  PageRank's scratch is fixed when the server starts; a member that
+outgrows it is pushed from the slabs.
 
 Each graph's requests are served in arrival order, so every request sees
 exactly the updates of its graph that arrived before it, whether it shares
